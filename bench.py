@@ -259,6 +259,8 @@ def row_kernel_name(N, C, adjoint=False):
             return ("k_row_pair_adj (adjoint RK4 row pass, both rates from one full-length complex transform, "
                     "update in registers)")
         return "k_row_pair (RK4 row pass, two components in full-length complex transforms, update in registers)"
+    if N <= 256:
+        return "k_lens_cluster (whole RK4 integration of a component map in one thread-block cluster)"
     return "k_row (RK4 row pass + fused epilogue)"
 
 
@@ -648,6 +650,8 @@ def main():
     peak_src = "measured" if "hbm_gbs" in peaks else "fallback"
 
     row_b = row_bytes_per_lens(C, n, P, 4, 4, adjoint=a.adjoint) * B / max(4 * n + 1, 1)  # per launch, all maps
+    if N <= 256:  # one launch per lens: the field in and out, the p planes once per component
+        row_b = (8 + 8 * (2 * n + 1)) * C * P * B
     col_b = col_bytes_per_lens(C, n, P) * B / max(4 * n, 1)
     kinds = {"row": (row_ms, row_n, row_b), "col": (col_ms, col_n, col_b)}
     dom = max(kinds, key=lambda k: kinds[k][0])

@@ -11,7 +11,7 @@
 #include <vector>
 
 #include "../../include/lenseflow.h"
-#include "lf_kernels.cuh"
+#include "lf_cluster.cuh"
 
 using namespace lf;
 
@@ -41,9 +41,12 @@ struct lf_plan_s {
   int device;
   void* tw;        // N complex values in the compute precision
   double2* tw64;   // N complex float64 (phi precompute)
-  void* twp;       // pass table of length N, then the column table, in the compute precision
+  void* twp;       // pass table of length N, the column table, the cluster kernels' table, in the compute precision
   const void* twc() const {  // the column table inside twp
     return static_cast<const char*>(twp) + (prec == LF_F64 ? sizeof(double2) : sizeof(float2)) * ptw_size(N);
+  }
+  const void* twg() const {  // the cluster kernels' table inside twp
+    return static_cast<const char*>(twc()) + (prec == LF_F64 ? sizeof(double2) : sizeof(float2)) * ctw_size(N);
   }
 };
 
@@ -79,6 +82,28 @@ static void fill_col_table(int L, Store store) {
       }
   }
 }
+
+// Pass table of the cluster kernels' group transforms (layout: cl_off_f3 / cl_off_i2 / cl_off_i3), E elements per lane.
+template <class Store>
+static void fill_cluster_table(int L, int E, Store store) {
+  if (!cl_tw_size(L, E)) return;
+  const int r2 = cl_r2(L, E), r3 = cl_r3(L, E);
+  const int blocks[4][3] = {
+      {r2, E, 0}, {r3, E * r2, cl_off_f3(L, E)}, {r2, r3, cl_off_i2(L, E)}, {E, L / E, cl_off_i3(L, E)}};
+  for (int b = 0; b < (cl_shared_table(L, E) ? 1 : 4); ++b) {
+    const int R = blocks[b][0], NS = blocks[b][1], off = blocks[b][2];
+    if (NS == 1) continue;  // a first pass has no twiddles
+    for (int r = 1; r < R; ++r)
+      for (int k = 0; k < NS; ++k) {
+        const double ang = -2.0 * M_PI * (double)r * (double)k / ((double)R * (double)NS);
+        store(off + (r - 1) * NS + k, std::cos(ang), std::sin(ang));
+      }
+  }
+}
+
+// elements per lane of the cluster kernels' transforms, and their table's entries
+static constexpr int cluster_e(int L, bool f64) { return f64 || L < 256 ? 8 : cl_elems<float, 256>(); }
+static constexpr int cluster_tw_entries(int L, bool f64) { return cl_tw_size(L, cluster_e(L, f64)); }
 
 namespace {
 
@@ -124,13 +149,14 @@ template <> struct Geo<double> {
 // entry point): the per-device high-water mark is an atomic, and a racing
 // thread at worst sets the same attribute twice.
 template <auto Kernel>
-cudaError_t ensure_smem(size_t smem) {
+cudaError_t ensure_smem(size_t smem, bool wide_cluster = false) {
   static std::atomic<size_t> done[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   if (done[dev].load(std::memory_order_relaxed) >= smem) return cudaSuccess;
   cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess && wide_cluster) e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e == cudaSuccess) {
     size_t cur = done[dev].load(std::memory_order_relaxed);
     while (cur < smem && !done[dev].compare_exchange_weak(cur, smem, std::memory_order_relaxed)) {
@@ -244,6 +270,15 @@ cudaError_t launch_col(int planes, cudaStream_t st, const StageArgs& a) {
   }
 }
 
+// p = M(t)^-1 grad(phi) at the 2n+1 times k / (2n), ascending, from the derivative planes
+template <typename T>
+cudaError_t run_p_planes(const StageArgs& a, int N, int B, int nsteps, cudaStream_t st) {
+  const long P = (long)N * N;
+  const int gx = (int)std::min<long>((P / 2 + 255) / 256, 1024);
+  return launch_k<k_p_planes<T>>(LF_KIND_PP, dim3(gx, B), 256, 0, st, reinterpret_cast<const T*>(a.phi),
+                                 reinterpret_cast<T*>(const_cast<void*>(a.pp)), P, 2 * nsteps + 1, 0.0, 0.5 / nsteps);
+}
+
 // The p planes hold p = M(t)^-1 grad(phi) at the 2n+1 times k / (2n), k = 0..2n, ascending; an
 // integration from t0 = 1 reads time t0 + k hh at index 2n - k.  ``pp_given``: the caller supplies
 // them (lf_lense_flow_pp), otherwise k_p_planes forms them from the derivative planes first.
@@ -262,12 +297,8 @@ cudaError_t run_lens_pp(const StageArgs& base, int B, int nsteps, double t0, dou
   const double hh = h / 2.0;
   if constexpr (PP) {
     a.pp_k = 2 * nsteps + 1;
-    if (!pp_given) {  // p at the times k / (2n), ascending
-      const long P = (long)N * N;
-      const int gx = (int)std::min<long>((P / 2 + 255) / 256, 1024);
-      e = launch_k<k_p_planes<T>>(LF_KIND_PP, dim3(gx, B), 256, 0, st, reinterpret_cast<const T*>(a.phi),
-                                  reinterpret_cast<T*>(const_cast<void*>(a.pp)), P, a.pp_k, 0.0,
-                                  0.5 / nsteps);
+    if (!pp_given) {
+      e = run_p_planes<T>(a, N, B, nsteps, st);
       if (e != cudaSuccess) return e;
     }
   }
@@ -327,13 +358,84 @@ cudaError_t run_lens_pp(const StageArgs& base, int B, int nsteps, double t0, dou
   return cudaSuccess;
 }
 
+// One cluster launch for the whole integration of every component of every map (N <= 256).
+template <typename T, int N, int CL, bool ADJ, bool PP, int MINB>
+cudaError_t launch_cluster(const StageArgs& a, int planes, int C, int nsteps, double t0, double t1, cudaStream_t st) {
+  using G = ClGeo<T, N, CL>;
+  constexpr auto kernel = k_lens_cluster<T, N, CL, ADJ, PP, MINB>;
+  constexpr size_t smem = sizeof(c2<T>) * (ClSystem<T, N, CL>::kElems + cl_tw_size(N, G::E)) + 32;  // + three mbarriers
+  cudaError_t e = ensure_smem<kernel>(smem, CL > 8);
+  if (e != cudaSuccess) return e;
+  ClusterArgs c;
+  std::memset(&c, 0, sizeof(c));
+  c.f_in = a.f_in;
+  c.f_out = a.f_out;
+  c.in_f64 = a.in_f64;
+  c.out_f64 = a.out_f64;
+  c.phi = a.phi;
+  c.pp = a.pp;
+  c.tw = a.twG;
+  c.kbase = a.kbase;
+  c.t0 = t0;
+  c.h = (t1 - t0) / nsteps;
+  c.nsteps = nsteps;
+  c.ncomp = C;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)planes * CL);
+  cfg.blockDim = dim3(G::NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CL;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  Prof* pf = (g_prof && g_prof->on) ? g_prof : nullptr;
+  cudaEvent_t e0 = pf ? pf->next() : nullptr, e1 = pf ? pf->next() : nullptr;
+  if (e0) cudaEventRecord(e0, st);
+  e = cudaLaunchKernelEx(&cfg, kernel, c);
+  if (e1) {
+    cudaEventRecord(e1, st);
+    pf->kind.push_back(LF_KIND_ROW);
+  }
+  return e;
+}
+
+// Blocks per cluster: as many as leave a block eight columns (64-byte puts), so that one map spreads over as
+// many SMs as it can.  Measured, one float32 lens of n = 7: T, one map, N = 64, 1, 2, 4 blocks 74, 59, 47 us;
+// N = 128, 4, 8 blocks 112, 74 us; N = 256, 8, 16 blocks 181, 130 us.  64 TQU maps, N = 64, 146, 107, 102 us;
+// N = 128, 531, 519 us; 48 QU maps, N = 256, 1,244, 1,063 us.  The sequence of 57 row and column passes that
+// this replaces took 183, 196 and 264 us for one map of the three sizes, 767 and 1,391 us for the last two
+// batches.  Larger maps do not fit a cluster's shared memory.
+template <typename T, int N, bool ADJ, bool PP>
+cudaError_t run_lens_cluster(const StageArgs& a, int B, int C, int nsteps, double t0, double t1, cudaStream_t st) {
+  constexpr int CL = N / 16;
+  constexpr int MINB = sizeof(T) == 8 ? 1 : 65536 / (ClGeo<T, N, CL>::NT * (N == 64 ? 168 : N == 128 ? 128 : 255));
+  return launch_cluster<T, N, CL, ADJ, PP, MINB>(a, B * C, C, nsteps, t0, t1, st);
+}
+
 // The p-plane path (a.pp set) is built for float32 plans only.
 template <typename T, int N, int C, bool ADJ>
 cudaError_t run_lens_n(const StageArgs& a, int B, int nsteps, double t0, double t1, cudaStream_t st, bool pp_given) {
-  if constexpr (std::is_same<T, float>::value) {
+  if constexpr (N <= 256) {
+    if constexpr (std::is_same<T, float>::value) {
+      if (a.pp) {
+        if (!pp_given) {
+          cudaError_t e = run_p_planes<T>(a, N, B, nsteps, st);
+          if (e != cudaSuccess) return e;
+        }
+        return run_lens_cluster<T, N, ADJ, true>(a, B, C, nsteps, t0, t1, st);
+      }
+    }
+    return run_lens_cluster<T, N, ADJ, false>(a, B, C, nsteps, t0, t1, st);
+  } else if constexpr (std::is_same<T, float>::value) {
     if (a.pp) return run_lens_pp<T, N, C, ADJ, true>(a, B, nsteps, t0, t1, st, pp_given);
+    return run_lens_pp<T, N, C, ADJ, false>(a, B, nsteps, t0, t1, st);
+  } else {
+    return run_lens_pp<T, N, C, ADJ, false>(a, B, nsteps, t0, t1, st);
   }
-  return run_lens_pp<T, N, C, ADJ, false>(a, B, nsteps, t0, t1, st);
 }
 
 template <typename T, int N>
@@ -836,7 +938,7 @@ int lf_plan_create(lf_plan_t* out, int nside, int ncomp, double pix_width, int p
     }
   }
   if (e == cudaSuccess) {
-    const size_t np = (size_t)ptw_size(nside) + (size_t)ctw_size(nside);
+    const size_t np = (size_t)ptw_size(nside) + (size_t)ctw_size(nside) + (size_t)cluster_tw_entries(nside, precision == LF_F64);
     std::vector<double2> pt(np);
     std::vector<float2> pt32(np);
     auto put = [&](int i, double c, double sn) {
@@ -845,6 +947,8 @@ int lf_plan_create(lf_plan_t* out, int nside, int ncomp, double pix_width, int p
     };
     fill_pass_table(nside, put);
     fill_col_table(nside, [&](int i, double c, double sn) { put(ptw_size(nside) + i, c, sn); });
+    fill_cluster_table(nside, cluster_e(nside, precision == LF_F64),
+                       [&](int i, double c, double sn) { put(ptw_size(nside) + ctw_size(nside) + i, c, sn); });
     const bool f64 = precision == LF_F64;
     const size_t bytes = f64 ? sizeof(double2) * np : sizeof(float2) * np;
     e = cudaMalloc(&p->twp, bytes);
@@ -976,6 +1080,7 @@ int lf_lense_flow(lf_plan_t p, const void* f_in, int in_dtype, void* f_out, int 
   a.twN = p->tw;
   a.twP = p->twp;
   a.twC = p->twc();
+  a.twG = p->twg();
   a.kbase = 2.0 * M_PI / ((double)p->N * p->pix_width);
   a.nplanes = batch * p->C;
   cudaError_t e;
@@ -1044,6 +1149,7 @@ int lf_lense_flow_pp(lf_plan_t p, const void* f_in, int in_dtype, void* f_out, i
   a.twN = p->tw;
   a.twP = p->twp;
   a.twC = p->twc();
+  a.twG = p->twg();
   a.kbase = 2.0 * M_PI / ((double)p->N * p->pix_width);
   a.nplanes = batch * p->C;
   g_prof = &p->prof;
@@ -1163,6 +1269,7 @@ int lf_lense_flow_vjp(lf_plan_t p, const void* f_lensed, const void* cotangent, 
   af.twN = p->tw;
   af.twP = p->twp;
   af.twC = p->twc();
+  af.twG = p->twg();
   af.kbase = 2.0 * M_PI / ((double)p->N * p->pix_width);
   af.nplanes = batch * p->C;
   af.grad = grad;
@@ -1232,6 +1339,7 @@ int lf_lense_flow_vjp_ckpt(lf_plan_t p, const void* f_in, const void* cotangent,
   af.twN = p->tw;
   af.twP = p->twp;
   af.twC = p->twc();
+  af.twG = p->twg();
   af.kbase = 2.0 * M_PI / ((double)p->N * p->pix_width);
   af.nplanes = batch * p->C;
   ad = af;
@@ -1320,8 +1428,8 @@ int lf_profile_read(lf_plan_t p, int kind, double* total_ms, int* launches) {
 // on the first call on the device, and only those addresses reach kernels.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[LF_NOALLOC_SCRATCH_BYTES];
 static __device__ __align__(256) float2 g_noalloc_tw[64 + 128 + 256 + 512 + 1024];
-// pass table + column table of every supported N, back to back
-constexpr int twp_entries(int n) { return ptw_size(n) + ctw_size(n); }
+// pass, column and cluster tables of every supported N, back to back
+constexpr int twp_entries(int n) { return ptw_size(n) + ctw_size(n) + cluster_tw_entries(n, false); }
 constexpr int kNoAllocTwp = twp_entries(64) + twp_entries(128) + twp_entries(256) + twp_entries(512) + twp_entries(1024);
 static __device__ __align__(256) float2 g_noalloc_twp[kNoAllocTwp];
 
@@ -1385,6 +1493,9 @@ int noalloc_setup(NoAllocDevice** out) {
       fill_col_table(n, [&](int i, double c, double sn) {
         host_p[off + ptw_size(n) + i] = make_float2((float)c, (float)sn);
       });
+      fill_cluster_table(n, cluster_e(n, false), [&](int i, double c, double sn) {
+        host_p[off + ptw_size(n) + ctw_size(n) + i] = make_float2((float)c, (float)sn);
+      });
     }
     e = cudaMemcpyToSymbol(g_noalloc_twp, host_p, sizeof(host_p));
     if (e != cudaSuccess) return cuda_status(e);
@@ -1440,6 +1551,7 @@ extern "C" int lf_lense_flow_noalloc(int nside, int ncomp, double pix_width, con
   a.twN = d->tw + noalloc_tw_offset(nside);
   a.twP = d->twp + noalloc_twp_offset(nside);
   a.twC = d->twp + noalloc_twp_offset(nside) + ptw_size(nside);
+  a.twG = d->twp + noalloc_twp_offset(nside) + ptw_size(nside) + ctw_size(nside);
   a.kbase = 2.0 * M_PI / ((double)nside * pix_width);
   a.nplanes = batch * ncomp;
   g_prof = nullptr;

@@ -40,6 +40,7 @@ struct StageArgs {
   const void* twN;  // N complex T, exp(-2 pi i k / N)
   const void* twP;  // pass table of length N (ptw_size(N) complex T): column pass, paired row pass
   const void* twC;  // column table of the two-pass column plan (ctw_size(N) complex T; N = 512)
+  const void* twG;  // table of the cluster kernels' group transforms (N <= 256)
   double kbase;     // 2 pi / (N d)
   double t_cur;     // time of the rate evaluated in this stage
   double t_next;    // time of the next stage input

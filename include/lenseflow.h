@@ -243,8 +243,9 @@ int lf_set_wait_polls(int polls);
 /* Launch timing for benchmarks and profiling.  While enabled, every kernel
  * launched through ``plan`` is bracketed by a CUDA event pair on its stream.
  * lf_profile_read synchronises on the last event and returns the summed
- * duration and count of the recorded launches of one kind.  No counterpart
- * in the reference (its device work is XLA-generated). */
+ * duration and count of the recorded launches of one kind.  LF_KIND_ROW: the
+ * row passes, or the kernels that integrate a whole lens (N <= 256).  No
+ * counterpart in the reference (its device work is XLA-generated). */
 
 enum lf_kernel_kind { LF_KIND_ROW = 0, LF_KIND_COL = 1, LF_KIND_PHI = 2, LF_KIND_PP = 3 };
 int lf_profile_enable(lf_plan_t plan, int enable);
