@@ -270,13 +270,13 @@ cudaError_t launch_col(int planes, cudaStream_t st, const StageArgs& a) {
   }
 }
 
-// p = M(t)^-1 grad(phi) at the 2n+1 times k / (2n), ascending, from the derivative planes
+// p = M(t)^-1 grad(phi) at the 2n+1 times t0 + k h / 2 from the derivative planes
 template <typename T>
-cudaError_t run_p_planes(const StageArgs& a, int N, int B, int nsteps, cudaStream_t st) {
+cudaError_t run_p_planes(const StageArgs& a, int N, int B, int nsteps, double t0, double h, cudaStream_t st) {
   const long P = (long)N * N;
   const int gx = (int)std::min<long>((P / 2 + 255) / 256, 1024);
   return launch_k<k_p_planes<T>>(LF_KIND_PP, dim3(gx, B), 256, 0, st, reinterpret_cast<const T*>(a.phi),
-                                 reinterpret_cast<T*>(const_cast<void*>(a.pp)), P, 2 * nsteps + 1, 0.0, 0.5 / nsteps);
+                                 reinterpret_cast<T*>(const_cast<void*>(a.pp)), P, 2 * nsteps + 1, t0, 0.5 * h);
 }
 
 // The p planes hold p = M(t)^-1 grad(phi) at the 2n+1 times k / (2n), k = 0..2n, ascending; an
@@ -298,7 +298,7 @@ cudaError_t run_lens_pp(const StageArgs& base, int B, int nsteps, double t0, dou
   if constexpr (PP) {
     a.pp_k = 2 * nsteps + 1;
     if (!pp_given) {
-      e = run_p_planes<T>(a, N, B, nsteps, st);
+      e = run_p_planes<T>(a, N, B, nsteps, 0.0, 1.0 / nsteps, st);
       if (e != cudaSuccess) return e;
     }
   }
@@ -358,31 +358,14 @@ cudaError_t run_lens_pp(const StageArgs& base, int B, int nsteps, double t0, dou
   return cudaSuccess;
 }
 
-// One cluster launch for the whole integration of every component of every map (N <= 256).
-template <typename T, int N, int CL, bool ADJ, bool PP, int MINB>
-cudaError_t launch_cluster(const StageArgs& a, int planes, int C, int nsteps, double t0, double t1, cudaStream_t st) {
-  using G = ClGeo<T, N, CL>;
-  constexpr auto kernel = k_lens_cluster<T, N, CL, ADJ, PP, MINB>;
-  constexpr size_t smem = sizeof(c2<T>) * (ClSystem<T, N, CL>::kElems + cl_tw_size(N, G::E)) + 32;  // + three mbarriers
-  cudaError_t e = ensure_smem<kernel>(smem, CL > 8);
+// A cluster launch of ``kernel`` on ``clusters`` clusters of CL blocks.
+template <auto Kernel, int CL, typename... Args>
+cudaError_t launch_clusters(long clusters, int nt, size_t smem, cudaStream_t st, Args... args) {
+  cudaError_t e = ensure_smem<Kernel>(smem, CL > 8);
   if (e != cudaSuccess) return e;
-  ClusterArgs c;
-  std::memset(&c, 0, sizeof(c));
-  c.f_in = a.f_in;
-  c.f_out = a.f_out;
-  c.in_f64 = a.in_f64;
-  c.out_f64 = a.out_f64;
-  c.phi = a.phi;
-  c.pp = a.pp;
-  c.tw = a.twG;
-  c.kbase = a.kbase;
-  c.t0 = t0;
-  c.h = (t1 - t0) / nsteps;
-  c.nsteps = nsteps;
-  c.ncomp = C;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)planes * CL);
-  cfg.blockDim = dim3(G::NT);
+  cfg.gridDim = dim3((unsigned)(clusters * CL));
+  cfg.blockDim = dim3(nt);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -395,12 +378,36 @@ cudaError_t launch_cluster(const StageArgs& a, int planes, int C, int nsteps, do
   Prof* pf = (g_prof && g_prof->on) ? g_prof : nullptr;
   cudaEvent_t e0 = pf ? pf->next() : nullptr, e1 = pf ? pf->next() : nullptr;
   if (e0) cudaEventRecord(e0, st);
-  e = cudaLaunchKernelEx(&cfg, kernel, c);
+  e = cudaLaunchKernelEx(&cfg, Kernel, args...);
   if (e1) {
     cudaEventRecord(e1, st);
     pf->kind.push_back(LF_KIND_ROW);
   }
   return e;
+}
+
+template <typename T, int N, int CL> constexpr size_t cluster_smem() {  // + three mbarriers
+  return sizeof(c2<T>) * (ClSystem<T, N, CL>::kElems + cl_tw_size(N, cl_elems<T, N>())) + 32;
+}
+
+inline ClusterArgs cluster_args(const StageArgs& a, int B, int C, int nsteps, double t0, double h) {
+  ClusterArgs c;
+  std::memset(&c, 0, sizeof(c));
+  c.f_in = a.f_in;
+  c.f_out = a.f_out;
+  c.in_f64 = a.in_f64;
+  c.out_f64 = a.out_f64;
+  c.phi = a.phi;
+  c.pp = a.pp;
+  c.tw = a.twG;
+  c.kbase = a.kbase;
+  c.t0 = t0;
+  c.h = h;
+  c.nsteps = nsteps;
+  c.ncomp = C;
+  c.rev = t0 != 0.0;  // p planes ascending from time 0
+  c.planes = (long)B * C;
+  return c;
 }
 
 // Blocks per cluster: as many as leave a block eight columns (64-byte puts), so that one map spreads over as
@@ -409,25 +416,71 @@ cudaError_t launch_cluster(const StageArgs& a, int planes, int C, int nsteps, do
 // N = 128, 531, 519 us; 48 QU maps, N = 256, 1,244, 1,063 us.  The sequence of 57 row and column passes that
 // this replaces took 183, 196 and 264 us for one map of the three sizes, 767 and 1,391 us for the last two
 // batches.  Larger maps do not fit a cluster's shared memory.
-template <typename T, int N, bool ADJ, bool PP>
-cudaError_t run_lens_cluster(const StageArgs& a, int B, int C, int nsteps, double t0, double t1, cudaStream_t st) {
-  constexpr int CL = N / 16;
-  constexpr int MINB = sizeof(T) == 8 ? 1 : 65536 / (ClGeo<T, N, CL>::NT * (N == 64 ? 168 : N == 128 ? 128 : 255));
-  return launch_cluster<T, N, CL, ADJ, PP, MINB>(a, B * C, C, nsteps, t0, t1, st);
+template <int N> constexpr int cluster_blocks() { return N / 16; }
+// resident blocks per SM that the register limit is set for (float64: whatever fits 255 registers)
+template <typename T, int N> constexpr int cluster_minb() {
+  return sizeof(T) == 8 ? 1 : 65536 / (ClGeo<T, N, cluster_blocks<N>()>::NT * (N == 64 ? 168 : N == 128 ? 128 : 255));
 }
 
-// The p-plane path (a.pp set) is built for float32 plans only.
+template <typename T, int N, bool ADJ, bool PP>
+cudaError_t run_lens_cluster(const StageArgs& a, int B, int C, int nsteps, double t0, double t1, cudaStream_t st,
+                             void* ckpt = nullptr) {
+  constexpr int CL = cluster_blocks<N>();
+  ClusterArgs c = cluster_args(a, B, C, nsteps, t0, (t1 - t0) / nsteps);
+  c.ckpt = ckpt;
+  return launch_clusters<k_lens_cluster<T, N, CL, ADJ, PP, cluster_minb<T, N>()>, CL>(
+      (long)B * C, ClGeo<T, N, CL>::NT, cluster_smem<T, N, CL>(), st, c);
+}
+
+// One step of a reverse pass on clusters: p at the step's three times (float32; into ``pp``, along ``f``),
+// ``f`` (standard) and ``d`` (adjoint) with their records, then the step's delta-phi terms.  The two systems run side by side unless one's output is the other's input (a
+// caller's buffers in a single-step pass): then one after the other, field first.
+template <typename T, int N, int C>
+cudaError_t run_vjp_step_cluster(ClusterArgs f, ClusterArgs d, void* pp, const void* phi, double* dacc, int B, int flip,
+                                 bool first, cudaStream_t st) {
+  constexpr int CL = cluster_blocks<N>();
+  constexpr auto kernel = k_vjp_step_cluster<T, N, CL, cluster_minb<T, N>()>;
+  const long P = (long)N * N, n = f.planes * P;
+  auto overlap = [n](const void* a, int a64, const void* b, int b64) {
+    const char *x = static_cast<const char*>(a), *y = static_cast<const char*>(b);
+    return x && x < y + n * (b64 ? 8 : 4) && y < x + n * (a64 ? 8 : 4);
+  };
+  cudaError_t e = cudaSuccess;
+  if constexpr (std::is_same<T, float>::value) {
+    StageArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.phi = phi;
+    a.pp = pp;
+    f.pp = d.pp = pp;
+    f.rev = 0;
+    d.rev = flip;
+    e = run_p_planes<T>(a, N, B, 1, f.t0, f.h, st);
+    if (e != cudaSuccess) return e;
+  }
+  const bool apart = overlap(d.f_out, d.out_f64, f.f_in, f.in_f64) || overlap(f.f_out, f.out_f64, d.f_in, d.in_f64);
+  e = launch_clusters<kernel, CL>((apart ? 1 : 2) * f.planes, ClGeo<T, N, CL>::NT, cluster_smem<T, N, CL>(),
+                                  st, f, d);
+  if (e == cudaSuccess && apart) {
+    ClusterArgs none = f;
+    none.planes = 0;
+    e = launch_clusters<kernel, CL>(d.planes, ClGeo<T, N, CL>::NT, cluster_smem<T, N, CL>(), st, none, d);
+  }
+  if (e != cudaSuccess) return e;
+  const int g = (int)std::min<long>(((long)B * P / 2 + 255) / 256, 148L * 8);
+  return launch<k_dphi_step<T, C>>(dim3(g), 256, 0, st, (const T*)f.save, (const T*)d.save, (const T*)phi, dacc, B, P,
+                                   d.t0, d.h, flip, (int)first);
+}
+
+// The p-plane path (a.pp set) is built for float32 plans, and for float64 ones of N <= 256.
 template <typename T, int N, int C, bool ADJ>
 cudaError_t run_lens_n(const StageArgs& a, int B, int nsteps, double t0, double t1, cudaStream_t st, bool pp_given) {
   if constexpr (N <= 256) {
-    if constexpr (std::is_same<T, float>::value) {
-      if (a.pp) {
-        if (!pp_given) {
-          cudaError_t e = run_p_planes<T>(a, N, B, nsteps, st);
-          if (e != cudaSuccess) return e;
-        }
-        return run_lens_cluster<T, N, ADJ, true>(a, B, C, nsteps, t0, t1, st);
+    if (a.pp) {
+      if (!pp_given) {
+        cudaError_t e = run_p_planes<T>(a, N, B, nsteps, 0.0, 1.0 / nsteps, st);
+        if (e != cudaSuccess) return e;
       }
+      return run_lens_cluster<T, N, ADJ, true>(a, B, C, nsteps, t0, t1, st);
     }
     return run_lens_cluster<T, N, ADJ, false>(a, B, C, nsteps, t0, t1, st);
   } else if constexpr (std::is_same<T, float>::value) {
@@ -650,6 +703,32 @@ cudaError_t run_vjp_n(const StageArgs& af0, const StageArgs& ad0, double* dacc, 
   const int gacc = (int)std::min<long>(((long)B * P + 255) / 256, 4096);
   StageArgs af = af0, ad = ad0;
   const double h = (t1 - t0) / nsteps;
+  if constexpr (N <= 256) {
+    // One cluster launch and one accumulation per step.  The records of a step's four stages take the twelve
+    // planes per component of the two systems, their gradients and stage input in the workspace.
+    const size_t plane = sizeof(T) * (size_t)B * C * P;
+    constexpr int io64 = std::is_same<T, double>::value;
+    ClusterArgs f = cluster_args(af0, B, C, 1, t0, h), d = cluster_args(ad0, B, C, 1, t0, h);
+    f.save = af0.y0;
+    d.save = static_cast<char*>(af0.y0) + 8 * plane;
+    void* pp = static_cast<char*>(ad0.between) + plane;
+    for (int i = 0; i < nsteps; ++i) {
+      const bool last = i == nsteps - 1;
+      f.t0 = d.t0 = t0 + i * h;
+      if (i > 0) {
+        f.f_in = af0.between;
+        d.f_in = ad0.between;
+        f.in_f64 = d.in_f64 = io64;
+      }
+      f.f_out = !last ? af0.between : af0.f_out == af0.between ? nullptr : af0.f_out;
+      d.f_out = !last ? ad0.between : ad0.f_out;
+      f.out_f64 = last ? af0.out_f64 : io64;
+      d.out_f64 = last ? ad0.out_f64 : io64;
+      cudaError_t e = run_vjp_step_cluster<T, N, C>(f, d, pp, af0.phi, dacc, B, 0, i == 0, st);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  } else {
   const double hh = h / 2.0;
   const double cw[4] = {1.0, 2.0, 2.0, 1.0};
   af.h = ad.h = h;
@@ -684,6 +763,7 @@ cudaError_t run_vjp_n(const StageArgs& af0, const StageArgs& ad0, double* dacc, 
     }
   }
   return cudaSuccess;
+  }
 }
 
 template <typename T, int N>
@@ -760,6 +840,41 @@ cudaError_t run_vjp_ckpt_n(const StageArgs& af0, const StageArgs& ad0, char* ckp
   const double cw[4] = {1.0, 2.0, 2.0, 1.0};
   StageArgs af = af0, ad = ad0;
   cudaError_t e;
+  if constexpr (N <= 256) {  // as run_vjp_n: the forward lens with its checkpoints, then two launches per step
+    constexpr int io64 = std::is_same<T, double>::value;
+    if (af.f_out == sink) af.f_out = nullptr;
+    // the p planes of the forward lens, if they fit what the reverse steps use later
+    if ((size_t)((char*)dacc - (char*)af.y0) >= sizeof(T) * 2 * (2 * (size_t)nsteps + 1) * P * B) {
+      af.pp = af.y0;
+      e = run_p_planes<T>(af, N, B, nsteps, 0.0, 1.0 / nsteps, st);
+      if (e != cudaSuccess) return e;
+      e = run_lens_cluster<T, N, false, true>(af, B, C, nsteps, t0, t1, st, ckpt);
+    } else {
+      e = run_lens_cluster<T, N, false, false>(af, B, C, nsteps, t0, t1, st, ckpt);
+    }
+    if (e != cudaSuccess) return e;
+    ClusterArgs f = cluster_args(af0, B, C, 1, t0, h), d = cluster_args(ad0, B, C, 1, t1, hb);
+    f.in_f64 = io64;
+    f.f_out = nullptr;
+    f.save = grads;
+    d.save = ad0.y0;
+    for (int ib = 0; ib < nsteps; ++ib) {
+      const int i = nsteps - 1 - ib;
+      const bool last = ib == nsteps - 1;
+      f.f_in = ckpt + (size_t)i * plane;
+      f.t0 = t0 + i * h;
+      d.t0 = t0 + (i + 1) * h;
+      if (ib > 0) {
+        d.f_in = ad0.between;
+        d.in_f64 = io64;
+      }
+      d.f_out = last ? ad0.f_out : ad0.between;
+      d.out_f64 = last ? ad0.out_f64 : io64;
+      e = run_vjp_step_cluster<T, N, C>(f, d, af0.between, af0.phi, dacc, B, 1, ib == 0, st);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  } else {
   // ---- forward integration, storing y_i at the start of each step
   af.h = h;
   af.stage = 0;
@@ -838,6 +953,7 @@ cudaError_t run_vjp_ckpt_n(const StageArgs& af0, const StageArgs& ad0, char* ckp
     }
   }
   return cudaSuccess;
+  }
 }
 
 template <typename T, int N>
@@ -979,10 +1095,10 @@ size_t lf_workspace_bytes(lf_plan_t p, int batch, int adjoint) {
   return el * (size_t)p->N * p->N * (size_t)batch * p->C * (adjoint ? 5 : 4);
 }
 
-// p-plane region: 2 (2n+1) planes per map, float32 plans only
+// p-plane region: 2 (2n+1) planes per map; float64 plans of N > 256 form p in the row passes
 static size_t pp_bytes(lf_plan_t p, int batch, int nsteps) {
-  if (p->prec != LF_F32 || nsteps <= 0) return 0;
-  return 4 * (size_t)p->N * p->N * (size_t)batch * 2 * (2 * (size_t)nsteps + 1);
+  if ((p->prec != LF_F32 && p->N > 256) || nsteps <= 0) return 0;
+  return (p->prec == LF_F64 ? 8 : 4) * (size_t)p->N * p->N * (size_t)batch * 2 * (2 * (size_t)nsteps + 1);
 }
 
 size_t lf_workspace_bytes_n(lf_plan_t p, int batch, int adjoint, int nsteps) {
@@ -1093,7 +1209,7 @@ int lf_lense_flow(lf_plan_t p, const void* f_in, int in_dtype, void* f_out, int 
 }
 
 size_t lf_pp_bytes(lf_plan_t p, int batch, int nsteps) {
-  if (!p || batch < 0 || nsteps < 1) return 0;
+  if (!p || batch < 0 || nsteps < 1 || p->prec != LF_F32) return 0;
   return pp_bytes(p, batch, nsteps);
 }
 
@@ -1283,6 +1399,8 @@ int lf_lense_flow_vjp(lf_plan_t p, const void* f_lensed, const void* cotangent, 
   ad.gx = ds + 4 * plane;
   ad.grad = nullptr;
   ad.dsave = dsave;
+  af.between = fback;
+  ad.between = spec;  // with p at one step's times behind it: the spectra are formed after the last step
   cudaStream_t st = (cudaStream_t)stream;
   g_prof = &p->prof;
   cudaError_t e = p->prec == LF_F64 ? run_vjp<double>(p->N, p->C, af, ad, dacc, batch, nsteps, t0, t1, st)
@@ -1351,6 +1469,8 @@ int lf_lense_flow_vjp_ckpt(lf_plan_t p, const void* f_in, const void* cotangent,
   ad.v = ds + 3 * plane;
   ad.gx = ds + 4 * plane;
   ad.dsave = dsave;
+  ad.between = dsave;
+  af.between = spec;  // p at one step's times
   cudaStream_t st = (cudaStream_t)stream;
   g_prof = &p->prof;
   cudaError_t e;

@@ -485,11 +485,15 @@ struct ClusterArgs {
   void* f_out;
   int in_f64, out_f64;
   const void* phi;  // derivative planes [B][5][N][N] of T
-  const void* pp;   // p planes [B][2n+1][2][N][N] of T, ascending in time (PP), else null
+  const void* pp;   // p planes [B][2n+1][2][N][N] of T (PP), else null
   const void* tw;   // cl_tw_size(N, E) complex T
   double kbase;     // 2 pi / (N d)
   double t0, h;     // start time and signed step
   int nsteps, ncomp;
+  int rev;          // time t0 + k h / 2 sits at p-plane index 2n - k instead of k
+  void* ckpt;       // null, or y at the start of every step, [n][B C][N][N] of T
+  void* save;       // SAVE (one step): of every stage, [4][B C] planes of T: d_x y, d_y y (standard) or y (adjoint)
+  long planes;      // B C
 };
 
 // One RK4 stage update (util.py:184-199) of a pixel: rate k of stage s; returns the next stage input.
@@ -502,11 +506,12 @@ template <typename T> __device__ __forceinline__ T rk4_update(int s, T k, T h, T
   return y0;
 }
 
-// ============================================================ the lens
-// grid: CL blocks (one cluster) per component of a map.  PP: p read from the p planes, else formed from the
-// derivative planes when the stage time changes.
-template <typename T, int N, int CL, bool ADJ, bool PP, int MINB>
-__global__ void __launch_bounds__(ClGeo<T, N, CL>::NT, MINB) k_lens_cluster(ClusterArgs a) {
+// ====================================================== the integration
+// One cluster integrates component plane ``cmap`` over a.nsteps steps.  PP: p read from the p planes, else
+// formed from the derivative planes when the stage time changes.  SAVE: the reverse passes' records of a
+// single step, the standard system's stage gradients or the adjoint one's stage inputs.
+template <typename T, int N, int CL, bool ADJ, bool PP, bool SAVE>
+__device__ __forceinline__ void cl_integrate(const ClusterArgs& a, long cmap) {
   using G = ClGeo<T, N, CL>;
   using S = ClSystem<T, N, CL>;
   constexpr int E = G::E, TP = G::TP;
@@ -520,7 +525,6 @@ __global__ void __launch_bounds__(ClGeo<T, N, CL>::NT, MINB) k_lens_cluster(Clus
   static_assert(TW * sizeof(c2<T>) % 16 == 0, "twiddle table: one bulk copy");
   const int tid = threadIdx.x;
   const uint32_t rank = CL > 1 ? cluster_rank() : 0u;
-  const long cmap = blockIdx.x / CL;  // component plane b C + c
   const long map = cmap / a.ncomp;
   S sys;
   sys.init(data, mbar + 1, tw, tid, rank);
@@ -538,12 +542,11 @@ __global__ void __launch_bounds__(ClGeo<T, N, CL>::NT, MINB) k_lens_cluster(Clus
   const T kx_scale = T(a.kbase / (double(N) * double(N)));
   const T hh = T(a.h);
   const int K = 2 * a.nsteps;
-  const bool rev = a.t0 != 0.0;  // time t0 + k h / 2 sits at p-plane index 2n - k
 
   T px[2][E], py[2][E];
   auto load_p = [&](int k) {  // p at time t0 + k h / 2 of this lane's pixels
     if constexpr (PP) {
-      const T* p = reinterpret_cast<const T*>(a.pp) + (map * (K + 1) + (rev ? K - k : k)) * 2 * P + r0 * N + lane;
+      const T* p = reinterpret_cast<const T*>(a.pp) + (map * (K + 1) + (a.rev ? K - k : k)) * 2 * P + r0 * N + lane;
 #pragma unroll
       for (int q = 0; q < 2; ++q)
 #pragma unroll
@@ -567,6 +570,14 @@ __global__ void __launch_bounds__(ClGeo<T, N, CL>::NT, MINB) k_lens_cluster(Clus
 
   T y0[2][E], acc[2][E];
   const long fo = cmap * P + r0 * N + lane;
+  auto store = [&](T* plane, const T (&v)[2][E]) {  // this lane's pixels of a plane of the component
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int e = 0; e < E; ++e) plane[r0 * N + lane + q * N + TP * e] = v[q][e];
+  };
+  T* save = reinterpret_cast<T*>(a.save) + cmap * P * (ADJ ? 1 : 2);
+  const long stage_planes = a.planes * P * (ADJ ? 1 : 2);
 #pragma unroll
   for (int q = 0; q < 2; ++q)
 #pragma unroll
@@ -576,6 +587,7 @@ __global__ void __launch_bounds__(ClGeo<T, N, CL>::NT, MINB) k_lens_cluster(Clus
       acc[q][e] = T(0);
     }
   int k_now = -1;
+  if constexpr (SAVE && ADJ) store(save, y0);
   cluster_sync<CL>();       // every block runs, with its barriers initialised, before anyone puts into it
   wait_or_record(mbar, 0);  // (a timed-out wait is recorded; the block goes on, as at every wait below)
   if constexpr (ADJ) {
@@ -593,6 +605,9 @@ __global__ void __launch_bounds__(ClGeo<T, N, CL>::NT, MINB) k_lens_cluster(Clus
     opaque(kxs);
     opaque(kys);
     const bool last = it == 4 * a.nsteps - 1;
+    if constexpr (!ADJ && !SAVE) {
+      if (s == 0 && a.ckpt) store(reinterpret_cast<T*>(a.ckpt) + ((it >> 2) * a.planes + cmap) * P, y0);
+    }
     sys.landed(0, it, polls, !last);
     // p at the rate's time (standard) or at the next stage's (adjoint), needed when the columns have landed
     const int k = ADJ ? i2 + (s < 2 ? 1 : 2) : i2 + (s == 0 ? 0 : s < 3 ? 1 : 2);
@@ -613,10 +628,21 @@ __global__ void __launch_bounds__(ClGeo<T, N, CL>::NT, MINB) k_lens_cluster(Clus
         yn[1][e] = rk4_update<T>(s, v[0][e].y, hh, y0[1][e], acc[1][e]);
       }
       if (last) break;
+      if constexpr (SAVE) store(save + (s + 1) * stage_planes, yn);
       sys.forward_adj(yn, px, py);
     } else {
       c2<T> v[2][E];
       sys.inverse_std(v, kys);
+      if constexpr (SAVE) {
+        T* gs = save + s * stage_planes + r0 * N + lane;
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            gs[q * N + TP * e] = v[q][e].x;
+            gs[P + q * N + TP * e] = v[q][e].y;
+          }
+      }
 #pragma unroll
       for (int q = 0; q < 2; ++q)
 #pragma unroll
@@ -627,6 +653,7 @@ __global__ void __launch_bounds__(ClGeo<T, N, CL>::NT, MINB) k_lens_cluster(Clus
     }
   }
   // (nothing is put into a block after its last Gx area has landed, so it may exit)
+  if (!a.f_out) return;
 #pragma unroll
   for (int q = 0; q < 2; ++q)
 #pragma unroll
@@ -635,6 +662,90 @@ __global__ void __launch_bounds__(ClGeo<T, N, CL>::NT, MINB) k_lens_cluster(Clus
       if (a.out_f64) reinterpret_cast<double*>(a.f_out)[i] = double(y0[q][e]);
       else reinterpret_cast<float*>(a.f_out)[i] = float(y0[q][e]);
     }
+}
+
+// The lens.  grid: one cluster per component of a map.
+template <typename T, int N, int CL, bool ADJ, bool PP, int MINB>
+__global__ void __launch_bounds__(ClGeo<T, N, CL>::NT, MINB) k_lens_cluster(ClusterArgs a) {
+  cl_integrate<T, N, CL, ADJ, PP, false>(a, blockIdx.x / CL);
+}
+
+// Measured, reference reverse pass of 16 TQU maps of 256^2, n = 7: row, column and accumulation launches per
+// stage 3.35 ms; per step, with p formed from the derivative planes 3.1 ms, read from p planes 2.0 ms.
+//
+// One RK4 step of the two systems of a reverse pass, with the records that k_dphi_step needs: the field
+// (standard) and the cotangent (adjoint), independent of one another within a step.  grid: two clusters per
+// component of a map.  p from the step's p planes; float64 forms it itself (no room for them in its workspace).
+template <typename T, int N, int CL, int MINB>
+__global__ void __launch_bounds__(ClGeo<T, N, CL>::NT, MINB) k_vjp_step_cluster(ClusterArgs f, ClusterArgs d) {
+  const long c = blockIdx.x / CL;
+  constexpr bool PP = sizeof(T) == 4;
+  if (c < f.planes) cl_integrate<T, N, CL, false, PP, true>(f, c);
+  else cl_integrate<T, N, CL, true, PP, true>(d, c - f.planes);
+}
+
+// delta-phi accumulation of one RK4 step from the records of its four stages: the rate of k_dphi_accum
+// (lense_flow.py:195-252) with the stage weights, summed in float64.  Adjoint stage j at time t + {0, 1/2,
+// 1/2, 1} h pairs with standard stage j, or with 3 - j where that system ran the other way (``flip``).  One
+// read and one write of the five accumulators per step instead of per stage, and the 2 x 2 inverse once per
+// distinct time: bound by its bytes, 57 us a step for 16 TQU maps of 256^2 (256 MB, 4.5 TB/s) against 4 x 25 us
+// by stages.  grads [4][B C][2][P], inputs [4][B C][P]; two pixels per thread.
+template <typename T, int C>
+__global__ void __launch_bounds__(256) k_dphi_step(const T* __restrict__ grads, const T* __restrict__ inputs,
+                                                   const T* __restrict__ phi, double* __restrict__ acc, int B, long P,
+                                                   double t, double h, int flip, int first) {
+  const long planes = (long)B * C, total = (long)B * P / 2;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+    const long b = 2 * i / P, px = 2 * i % P;
+    const T* ph = phi + b * 5 * P + px;
+    c2<T> g[5];
+#pragma unroll
+    for (int j = 0; j < 5; ++j) g[j] = *reinterpret_cast<const c2<T>*>(ph + j * P);
+    double sum[5][2] = {};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {  // the distinct times: adjoint stages {0}, {1, 2}, {3}
+      double f[2][2] = {};         // fdf = sum of weight x delta x gradient, (x, y) of the two pixels
+#pragma unroll
+      for (int j = k == 0 ? 0 : 2 * k - 1; j <= (k == 0 ? 0 : k == 1 ? 2 : 3); ++j) {
+        const double w = k == 1 ? 2.0 : 1.0;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const long pl = b * C + c;
+          const c2<T> d = *reinterpret_cast<const c2<T>*>(inputs + (j * planes + pl) * P + px);
+          const T* gp = grads + ((flip ? 3 - j : j) * planes + pl) * 2 * P + px;
+          const c2<T> gx = *reinterpret_cast<const c2<T>*>(gp), gy = *reinterpret_cast<const c2<T>*>(gp + P);
+          f[0][0] += w * double(d.x) * double(gx.x);
+          f[0][1] += w * double(d.x) * double(gy.x);
+          f[1][0] += w * double(d.y) * double(gx.y);
+          f[1][1] += w * double(d.y) * double(gy.y);
+        }
+      }
+      const double tt = t + 0.5 * k * h;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const double gx = q ? g[0].y : g[0].x, gy = q ? g[1].y : g[1].x, gxx = q ? g[2].y : g[2].x,
+                     gxy = q ? g[3].y : g[3].x, gyy = q ? g[4].y : g[4].x;
+        const double mxx = 1.0 + tt * gxx, mxy = tt * gxy, myy = 1.0 + tt * gyy;
+        const double inv = 1.0 / (mxx * myy - mxy * mxy + 1e-12);
+        const double ixx = myy * inv, ixy = -mxy * inv, iyy = mxx * inv;
+        const double ax = ixx * f[q][0] + ixy * f[q][1], ay = ixy * f[q][0] + iyy * f[q][1];
+        const double pxv = gx * ixx + gy * ixy, pyv = gx * ixy + gy * iyy;
+        sum[0][q] += ax;
+        sum[1][q] += ay;
+        sum[2][q] += tt * pxv * ax;
+        sum[3][q] += tt * (pxv * ay + pyv * ax);
+        sum[4][q] += tt * pyv * ay;
+      }
+    }
+    const double w6 = h / 6.0;
+    double* o = acc + b * 5 * P + px;
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+      double2* oj = reinterpret_cast<double2*>(o + j * P);
+      const double2 old = first ? make_double2(0.0, 0.0) : *oj;
+      *oj = make_double2(old.x + w6 * sum[j][0], old.y + w6 * sum[j][1]);
+    }
+  }
 }
 
 }  // namespace lf

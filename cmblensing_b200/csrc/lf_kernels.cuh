@@ -51,6 +51,7 @@ struct StageArgs {
   // reverse-mode (VJP) extras
   void* grad;       // standard pass with SAVE: d_x y_s, d_y y_s, [B*C][2][N][N] T
   void* dsave;      // adjoint pass with SAVE: next stage input, [B*C][N][N] T
+  void* between;    // reverse pass on clusters (N <= 256): fields between steps, p planes of a step
   // p = M(t)^-1 grad(phi) at the 2n+1 stage times t0 + k h/2 (row pass with PP):
   // [B][pp_k][2][N][N] T; this stage reads time index pp_idx
   const void* pp;

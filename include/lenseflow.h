@@ -62,7 +62,8 @@ int lf_plan_destroy(lf_plan_t plan);
 
 /* Bytes of caller workspace needed by lf_lense_flow for ``batch`` maps. */
 size_t lf_workspace_bytes(lf_plan_t plan, int batch, int adjoint);
-/* Workspace with which lf_lense_flow of a float32 plan also precomputes
+/* Workspace with which lf_lense_flow of a float32 plan, or of a float64 one
+ * with N <= 256, also precomputes
  * p = M(t)^-1 grad(phi) at the 2 nsteps + 1 RK4 stage times (lense_flow.py:
  * 373-381, :398-415; two planes per time and map) so that every row pass
  * reads two planes per pixel instead of five.  lf_lense_flow takes that path

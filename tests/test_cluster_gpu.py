@@ -70,3 +70,54 @@ def test_more_clusters_than_fit_and_two_streams(torch_cuda, N, B):
         for i in range(B):
             assert torch.equal(out[i], alone[reps[i]][0]), i
     assert engine.wait_timeouts() == 0
+
+
+def _grad_problem(torch, N, C, B, n):
+    from cmblensing_b200 import engine
+    from cmblensing_b200.simulate import lens_batch
+    f, phis = lens_batch(N, 3.0, B, C, seed0=110)
+    pw = R.pix_width_of(3.0)
+    cot = np.random.default_rng(111).standard_normal(f.shape)
+    out = {}
+    for prec in ("f32", "f64"):
+        plan = engine.get_plan(N, C, pw, prec)
+        planes = plan.phi_planes(torch.as_tensor(phis, device="cuda"))
+        out[prec] = (plan, planes, torch.as_tensor(f, device="cuda", dtype=plan.dtype),
+                     torch.as_tensor(cot, device="cuda", dtype=plan.dtype))
+    return out
+
+
+@pytest.mark.parametrize("N,C,n", [(64, 1, 1), (64, 3, 2), (128, 2, 1), (128, 1, 14), (256, 3, 1), (256, 2, 3)])
+@pytest.mark.parametrize("scheme", ["reference", "exact"])
+def test_reverse_passes_float32_against_float64(torch_cuda, N, C, n, scheme):
+    """Both reverse schemes, one launch pair per RK4 step, at the edges of their step counts (a single step; more
+    steps than the forward lens's p planes find room for): float32 within the engine's gradient tolerance 2e-5 of
+    the float64 engine, which the oracle pins (test_vjp_gpu)."""
+    torch = torch_cuda
+    got = {}
+    for prec, (plan, planes, f, cot) in _grad_problem(torch, N, C, 2, n).items():
+        fn = plan.lense_flow_vjp_ckpt if scheme == "exact" else plan.lense_flow_vjp
+        got[prec] = [x.cpu().numpy() for x in fn(f, cot, planes, n, phi_basis="map")] + \
+                    [x.cpu().numpy() for x in fn(f, cot, planes, n, -1, "fourier", True)]
+    for a, b in zip(got["f32"], got["f64"]):
+        assert rel_l2(a, b) < 2e-5
+
+
+def test_single_step_reverse_pass_in_place(torch_cuda):
+    """A one-step reverse pass whose delta-f overwrites the lensed field it reads: as with separate buffers."""
+    import ctypes
+    torch = torch_cuda
+    from cmblensing_b200 import _native as nat
+    N, C, B = 64, 2, 5
+    plan, planes, f, cot = _grad_problem(torch, N, C, B, 1)["f32"]
+    df, dphi = plan.lense_flow_vjp(f, cot, planes, 1)
+    g = f.clone()
+    dphi2 = torch.empty_like(dphi)
+    nbytes = plan._lib.lf_vjp_workspace_bytes(plan.handle, B)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    nat.check(plan._lib.lf_lense_flow_vjp(plan.handle, ptr(g), ptr(cot), nat.LF_F32, ptr(planes), B, 1, 1, ptr(g), None,
+                                          ptr(dphi2), nat.LF_PHI_FOURIER, ptr(ws), nbytes,
+                                          ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    assert torch.equal(g, df) and torch.equal(dphi2, dphi)
