@@ -261,7 +261,7 @@ def row_kernel_name(N, C, adjoint=False):
         return "k_row_pair (RK4 row pass, two components in full-length complex transforms, update in registers)"
     if N <= 256:
         return "k_lens_cluster (whole RK4 integration of a component map in one thread-block cluster)"
-    return "k_row (RK4 row pass + fused epilogue)"
+    return "k_row_rows (RK4 row pass of row pairs of one component, update in registers)"
 
 
 def col_bytes_per_lens(C, n, P):

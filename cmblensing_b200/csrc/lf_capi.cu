@@ -45,6 +45,9 @@ struct lf_plan_s {
   const void* twc() const {  // the column table inside twp
     return static_cast<const char*>(twp) + (prec == LF_F64 ? sizeof(double2) : sizeof(float2)) * ptw_size(N);
   }
+  const void* twr() const {  // the row-pair table inside twp (N = 512, 1024)
+    return static_cast<const char*>(twc()) + (prec == LF_F64 ? sizeof(double2) : sizeof(float2)) * ctw_size(N);
+  }
   const void* twg() const {  // the cluster kernels' table inside twp
     return static_cast<const char*>(twc()) + (prec == LF_F64 ? sizeof(double2) : sizeof(float2)) * ctw_size(N);
   }
@@ -81,6 +84,20 @@ static void fill_col_table(int L, Store store) {
         store(off + (r - 1) * NS + k, std::cos(ang), std::sin(ang));
       }
   }
+}
+
+// Table of the row-pair pass (layout: block (rtw_mid, 8), then block (8, L / 8)).
+static constexpr int row_tw_entries(int L) { return L == 512 || L == 1024 ? rtw_size(L) : 0; }
+template <class Store>
+static void fill_row_table(int L, Store store) {
+  if (!row_tw_entries(L)) return;
+  const int blocks[2][3] = {{rtw_mid(L), 8, 0}, {8, L / 8, (rtw_mid(L) - 1) * 8}};
+  for (const auto& b : blocks)
+    for (int r = 1; r < b[0]; ++r)
+      for (int k = 0; k < b[1]; ++k) {
+        const double ang = -2.0 * M_PI * (double)r * (double)k / ((double)b[0] * (double)b[1]);
+        store(b[2] + (r - 1) * b[1] + k, std::cos(ang), std::sin(ang));
+      }
 }
 
 // Pass table of the cluster kernels' group transforms (layout: cl_off_f3 / cl_off_i2 / cl_off_i3), E elements per lane.
@@ -305,6 +322,7 @@ cudaError_t run_lens_pp(const StageArgs& base, int B, int nsteps, double t0, dou
   const bool rev = t0 != 0.0;  // time t0 + k hh sits at index 2n - k
   auto pidx = [=](int k) { return rev ? 2 * nsteps - k : k; };
   a.h = h;
+  a.ncomp = C;
   a.stage = 0;
   a.last = 0;
   a.t_cur = t0;
@@ -349,6 +367,11 @@ cudaError_t run_lens_pp(const StageArgs& base, int B, int nsteps, double t0, dou
         constexpr int PL = 2, PNT = (N / 8) * PL;
         e = launch_k<k_row_pair_adj<N, PL, PNT, 6>>(LF_KIND_ROW, dim3(N / PL, B), PNT,
                                                     row_pair_smem_bytes<PL>(N), st, a);
+      } else if constexpr (PP && std::is_same<T, float>::value) {
+        // other shapes with p planes: row pairs of one component, 128 threads, five blocks per SM
+        constexpr int PL = 1024 / N, PNT = (N / 8) * PL;
+        e = launch_k<k_row_rows<N, PL, PNT, 5, ADJ>>(LF_KIND_ROW, dim3(N / (2 * PL), B * C), PNT,
+                                                     row_rows_smem_bytes<N, PL>(), st, a);
       } else {
         e = launch_k<k_row<T, N, C, ADJ, false, RL, RNT, false, RMB, PP>>(LF_KIND_ROW, grow, RNT, smem_row, st, a);
       }
@@ -1054,7 +1077,8 @@ int lf_plan_create(lf_plan_t* out, int nside, int ncomp, double pix_width, int p
     }
   }
   if (e == cudaSuccess) {
-    const size_t np = (size_t)ptw_size(nside) + (size_t)ctw_size(nside) + (size_t)cluster_tw_entries(nside, precision == LF_F64);
+    const size_t np = (size_t)ptw_size(nside) + (size_t)ctw_size(nside) + (size_t)row_tw_entries(nside) +
+                      (size_t)cluster_tw_entries(nside, precision == LF_F64);
     std::vector<double2> pt(np);
     std::vector<float2> pt32(np);
     auto put = [&](int i, double c, double sn) {
@@ -1063,6 +1087,7 @@ int lf_plan_create(lf_plan_t* out, int nside, int ncomp, double pix_width, int p
     };
     fill_pass_table(nside, put);
     fill_col_table(nside, [&](int i, double c, double sn) { put(ptw_size(nside) + i, c, sn); });
+    fill_row_table(nside, [&](int i, double c, double sn) { put(ptw_size(nside) + ctw_size(nside) + i, c, sn); });
     fill_cluster_table(nside, cluster_e(nside, precision == LF_F64),
                        [&](int i, double c, double sn) { put(ptw_size(nside) + ctw_size(nside) + i, c, sn); });
     const bool f64 = precision == LF_F64;
@@ -1196,6 +1221,7 @@ int lf_lense_flow(lf_plan_t p, const void* f_in, int in_dtype, void* f_out, int 
   a.twN = p->tw;
   a.twP = p->twp;
   a.twC = p->twc();
+  a.twR = p->twr();
   a.twG = p->twg();
   a.kbase = 2.0 * M_PI / ((double)p->N * p->pix_width);
   a.nplanes = batch * p->C;
@@ -1265,6 +1291,7 @@ int lf_lense_flow_pp(lf_plan_t p, const void* f_in, int in_dtype, void* f_out, i
   a.twN = p->tw;
   a.twP = p->twp;
   a.twC = p->twc();
+  a.twR = p->twr();
   a.twG = p->twg();
   a.kbase = 2.0 * M_PI / ((double)p->N * p->pix_width);
   a.nplanes = batch * p->C;
@@ -1549,7 +1576,7 @@ int lf_profile_read(lf_plan_t p, int kind, double* total_ms, int* launches) {
 static __device__ __align__(256) unsigned char g_noalloc_scratch[LF_NOALLOC_SCRATCH_BYTES];
 static __device__ __align__(256) float2 g_noalloc_tw[64 + 128 + 256 + 512 + 1024];
 // pass, column and cluster tables of every supported N, back to back
-constexpr int twp_entries(int n) { return ptw_size(n) + ctw_size(n) + cluster_tw_entries(n, false); }
+constexpr int twp_entries(int n) { return ptw_size(n) + ctw_size(n) + row_tw_entries(n) + cluster_tw_entries(n, false); }
 constexpr int kNoAllocTwp = twp_entries(64) + twp_entries(128) + twp_entries(256) + twp_entries(512) + twp_entries(1024);
 static __device__ __align__(256) float2 g_noalloc_twp[kNoAllocTwp];
 
@@ -1613,6 +1640,9 @@ int noalloc_setup(NoAllocDevice** out) {
       fill_col_table(n, [&](int i, double c, double sn) {
         host_p[off + ptw_size(n) + i] = make_float2((float)c, (float)sn);
       });
+      fill_row_table(n, [&](int i, double c, double sn) {
+        host_p[off + ptw_size(n) + ctw_size(n) + i] = make_float2((float)c, (float)sn);
+      });
       fill_cluster_table(n, cluster_e(n, false), [&](int i, double c, double sn) {
         host_p[off + ptw_size(n) + ctw_size(n) + i] = make_float2((float)c, (float)sn);
       });
@@ -1671,7 +1701,7 @@ extern "C" int lf_lense_flow_noalloc(int nside, int ncomp, double pix_width, con
   a.twN = d->tw + noalloc_tw_offset(nside);
   a.twP = d->twp + noalloc_twp_offset(nside);
   a.twC = d->twp + noalloc_twp_offset(nside) + ptw_size(nside);
-  a.twG = d->twp + noalloc_twp_offset(nside) + ptw_size(nside) + ctw_size(nside);
+  a.twR = a.twG = d->twp + noalloc_twp_offset(nside) + ptw_size(nside) + ctw_size(nside);
   a.kbase = 2.0 * M_PI / ((double)nside * pix_width);
   a.nplanes = batch * ncomp;
   g_prof = nullptr;

@@ -40,6 +40,7 @@ struct StageArgs {
   const void* twN;  // N complex T, exp(-2 pi i k / N)
   const void* twP;  // pass table of length N (ptw_size(N) complex T): column pass, paired row pass
   const void* twC;  // column table of the two-pass column plan (ctw_size(N) complex T; N = 512)
+  const void* twR;  // table of the row-pair passes (rtw_size(N) complex T; N = 512, 1024)
   const void* twG;  // table of the cluster kernels' group transforms (N <= 256)
   double kbase;     // 2 pi / (N d)
   double t_cur;     // time of the rate evaluated in this stage
@@ -48,6 +49,7 @@ struct StageArgs {
   int stage;        // 1..4 (0 = init)
   int last;         // final stage of the integration
   int nplanes;      // B*C (column pass)
+  int ncomp;        // C (row-pair pass)
   // reverse-mode (VJP) extras
   void* grad;       // standard pass with SAVE: d_x y_s, d_y y_s, [B*C][2][N][N] T
   void* dsave;      // adjoint pass with SAVE: next stage input, [B*C][N][N] T
@@ -899,6 +901,221 @@ __global__ void __launch_bounds__(NT, MINB) k_row_pair_adj(StageArgs a) {
     void* dst = which == 0 ? a.s : a.v;
     st2<T>(spec(dst, 0) + rw * H + 2 * t, s0);
     st2<T>(spec(dst, 1) + rw * H + 2 * t, s1);
+  }
+}
+
+// ============================================ row pass, row pairs
+// The RK4 stage update of one component with the p planes, N = 512 or 1024, FP32, any number of components
+// (each component plane has its own blocks).  As k_row_pair, with two rows in the place of two components:
+// standard RHS, Z = DX + i DY per row (inverse) and w = y_a + i y_b per row pair (forward); adjoint RHS, one
+// inverse transform of Z = K_a + i K_b per pair and w = (p_x + i p_y) y per row (forward), whose split gives
+// U and V.  Same staging by bulk copies, register passes and bounded waits.  A block holds 2 LINES rows: tile
+// q its rows [q LINES, (q + 1) LINES), pairs (line, LINES + line).  Radices 8 x 8 x 8 or 8 x 16 x 8, so that
+// the inverse's last and the forward's first pass see the same eight elements of a row.
+// Against the general row pass (half-length transforms with real-FFT passes around them in shared memory) it
+// is bound by its bytes instead of by instructions and latency: one lens, n = 7, 3 TQU maps of 1024^2 4,084 ->
+// 2,344 us (adjoint 4,448 -> 2,501), 8 TQU maps of 512^2 1,929 -> 1,356 (2,054 -> 1,370), 16 T maps of 512^2
+// 1,151 -> 895.  A single T map of 512^2 (384, 387 us) is bound by the latency of its launches either way.
+__host__ __device__ constexpr int rtw_mid(int n) { return n / 64; }  // radix of the middle pass
+__host__ __device__ constexpr int rtw_size(int n) { return (rtw_mid(n) - 1) * 8 + 7 * (n / 8); }
+
+template <int N, int LINES> constexpr size_t row_rows_smem_bytes() {
+  return sizeof(float2) * (rtw_size(N) + 2 * LINES * N) + sizeof(float) * 4 * LINES * N + 16;
+}
+
+template <int N, int LINES, int NT, int MINB, bool ADJ>
+__global__ void __launch_bounds__(NT, MINB) k_row_rows(StageArgs a) {
+  using T = float;
+  constexpr int H = N / 2;
+  constexpr long P = (long)N * N;
+  constexpr int R = 8, NB = N / R, RM = rtw_mid(N);
+  static_assert(N == 512 || N == 1024, "radix 8 x 8 x 8 or 8 x 16 x 8");
+  static_assert(NB * LINES == NT, "one (row pair, butterfly) per thread in the fused passes");
+  constexpr int TILE = LINES * N;
+  constexpr int RB = 2 * LINES * N;                  // floats of the block's rows
+  constexpr int NTI = ADJ ? 1 : 2, NTO = ADJ ? 2 : 1;  // tiles of the inverse and of the forward transforms
+  constexpr int IT = LINES * (H / 2) / NT;           // packed element pairs per row pair and thread in the load phase
+  static_assert(LINES * (H / 2) % NT == 0, "whole load-phase iterations");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  c2<T>* tw = reinterpret_cast<c2<T>*>(smem_raw);
+  c2<T>* buf = tw + rtw_size(N);                     // tile q at buf + q * TILE
+  T* stg = reinterpret_cast<T*>(buf + 2 * TILE);     // y0, then acc, of the block's rows
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(stg + 2 * RB);  // [0]: staged update operands, [1]: spectra
+  const int tid = threadIdx.x;
+  const int r0 = blockIdx.x * 2 * LINES;
+  const long plane = blockIdx.y, map = plane / a.ncomp;
+  const long prow0 = (long)r0 * N;
+  const bool with_acc = a.stage > 1;
+  auto spec = [&](void* base) { return reinterpret_cast<c2<T>*>(base) + plane * (N * (long)H) + (long)r0 * H; };
+  static_assert(rtw_size(N) * sizeof(c2<T>) % 16 == 0, "pass table: one bulk copy");
+  pdl_launch_dependents();
+  if (tid == 0) {
+    mbar_init(mbar, 1);
+    mbar_init(mbar + 1, 1);
+    mbar_expect_tx(mbar + 1, uint32_t(rtw_size(N) * sizeof(c2<T>) + 4 * LINES * H * sizeof(c2<T>)));
+    bulk_g2s(tw, a.twR, rtw_size(N) * sizeof(c2<T>), mbar + 1);
+    pdl_wait();  // the other copies read what the previous kernel wrote
+    for (int q = 0; q < 2; ++q) {  // Gx, then S (adjoint: V), of the tile's rows, packed
+      bulk_g2s(buf + q * TILE, spec(a.gx) + q * LINES * H, LINES * H * sizeof(c2<T>), mbar + 1);
+      bulk_g2s(buf + q * TILE + LINES * H, spec(ADJ ? a.v : a.s) + q * LINES * H, LINES * H * sizeof(c2<T>), mbar + 1);
+    }
+    mbar_expect_tx(mbar, uint32_t((with_acc ? 2 : 1) * RB * sizeof(T)));
+    bulk_g2s(stg, reinterpret_cast<const T*>(a.y0) + plane * P + prow0, RB * sizeof(T), mbar);
+    if (with_acc) bulk_g2s(stg + RB, reinterpret_cast<const T*>(a.acc) + plane * P + prow0, RB * sizeof(T), mbar);
+  }
+  pdl_wait();  // every thread, before its own global reads and writes
+  const int j = tid % NB, line = tid / NB;
+  T px[2][R], py[2][R];  // p (adjoint: at the next stage's time) of the thread's pixels, hidden under the transforms
+  {
+    const T* pq = reinterpret_cast<const T*>(a.pp) + (map * a.pp_k + a.pp_idx) * 2 * P + prow0 + line * N + j;
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        px[q][r] = __ldg(pq + q * LINES * N + NB * r);
+        py[q][r] = __ldg(pq + P + q * LINES * N + NB * r);
+      }
+  }
+  const c2<T>* tw2 = tw;                      // (RM, 8)
+  const c2<T>* tw3 = tw + (RM - 1) * 8;       // (8, N / 8)
+  const T ky_scale = T(a.kbase / double(N));
+  __syncthreads();  // barriers initialised before anyone waits on them
+  // a timed-out wait is recorded and the block goes on, so that every thread meets every barrier below
+  wait_or_record(mbar + 1, 0);
+
+  // ------------- load: the packed rows sit in the tiles; all of them are read before Z overwrites them
+  c2<T> gv[2][IT][2], sv[2][IT][2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+      const int idx = tid + it * NT, t = idx % (H / 2), row = idx / (H / 2);
+      ld2<T>(buf + q * TILE + row * H + 2 * t, gv[q][it]);
+      ld2<T>(buf + q * TILE + LINES * H + row * H + 2 * t, sv[q][it]);
+    }
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int idx = tid + it * NT, t = idx % (H / 2), row = idx / (H / 2);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int k = 2 * t + e;
+      const T f = ky_scale * T(k);
+      if constexpr (ADJ) {
+        if (k == 0) {  // real DC and Nyquist bins of each rate; i KY contributes nothing there
+          buf[sw<T, LINES>(0, row)] = mk<T>(gv[0][it][0].x, gv[1][it][0].x);
+          buf[sw<T, LINES>(H, row)] = mk<T>(gv[0][it][0].y, gv[1][it][0].y);
+        } else {
+          const c2<T> k0 = mk<T>(gv[0][it][e].x - f * sv[0][it][e].y, gv[0][it][e].y + f * sv[0][it][e].x);
+          const c2<T> k1 = mk<T>(gv[1][it][e].x - f * sv[1][it][e].y, gv[1][it][e].y + f * sv[1][it][e].x);
+          buf[sw<T, LINES>(k, row)] = mk<T>(k0.x - k1.y, k0.y + k1.x);      // K_a + i K_b
+          buf[sw<T, LINES>(N - k, row)] = mk<T>(k0.x + k1.y, k1.x - k0.y);  // conj(K_a) + i conj(K_b)
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          c2<T>* z = buf + q * TILE;
+          const c2<T> g = gv[q][it][e], sq = sv[q][it][e];
+          if (k == 0) {
+            z[sw<T, LINES>(0, row)] = mk<T>(g.x, T(0));
+            z[sw<T, LINES>(H, row)] = mk<T>(g.y, T(0));
+          } else {
+            z[sw<T, LINES>(k, row)] = mk<T>(g.x - f * sq.x, g.y - f * sq.y);       // DX + i DY, DY = i f S
+            z[sw<T, LINES>(N - k, row)] = mk<T>(g.x + f * sq.x, -g.y - f * sq.y);  // conj(DX) + i conj(DY)
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  stockham_pass<T, N, R, 1, LINES, NTI, NT, true, N, true>(buf, tw, tid);
+  stockham_pass<T, N, RM, R, LINES, NTI, NT, true, N, true>(buf, tw2, tid);
+
+  // ----------------- inverse pass 3 -> RK4 update -> forward pass 1, in registers
+  c2<T> v[2][R];
+#pragma unroll
+  for (int q = 0; q < NTI; ++q)
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[q][r] = buf[q * TILE + sw<T, LINES>(j + r * NB, line)];
+#pragma unroll
+  for (int r = 1; r < R; ++r) {
+    const c2<T> w = tw3[(r - 1) * NB + j];  // W_N^(r j): NS = N / R
+#pragma unroll
+    for (int q = 0; q < NTI; ++q) v[q][r] = twmul<T, true>(v[q][r], w);
+  }
+#pragma unroll
+  for (int q = 0; q < NTI; ++q) dft<R, T, true>(v[q]);
+  // standard: v[q][r] = dx + i dy at pixel n = j + NB r of row q; adjoint: v[0][r] = (k_a, k_b)
+  if (!wait_or_record(mbar, 0)) return;  // the staged operands: recorded, drained, leave
+  const T hh = T(a.h);
+  c2<T> w[2][R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    T yn[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int n = (q * LINES + line) * N + j + NB * r;  // within the block's rows
+      const T k = ADJ ? (q == 0 ? v[0][r].x : v[0][r].y) : px[q][r] * v[q][r].x + py[q][r] * v[q][r].y;
+      const T y0 = stg[n];
+      T* accg = reinterpret_cast<T*>(a.acc) + plane * P + prow0;
+      if (a.stage == 1) {
+        yn[q] = y0 + T(0.5) * hh * k;
+        accg[n] = k;
+      } else if (a.stage < 4) {
+        yn[q] = y0 + (a.stage == 2 ? T(0.5) * hh : hh) * k;
+        accg[n] = stg[RB + n] + T(2) * k;
+      } else {
+        yn[q] = y0 + hh / T(6) * (stg[RB + n] + k);
+        const long fo = plane * P + prow0 + n;
+        if (!a.last) reinterpret_cast<T*>(a.y0)[fo] = yn[q];
+        else if (a.out_f64) reinterpret_cast<double*>(a.f_out)[fo] = double(yn[q]);
+        else reinterpret_cast<float*>(a.f_out)[fo] = yn[q];
+      }
+      if constexpr (ADJ) w[q][r] = mk<T>(px[q][r] * yn[q], py[q][r] * yn[q]);
+    }
+    if constexpr (!ADJ) w[0][r] = mk<T>(yn[0], yn[1]);
+  }
+  if (a.last) return;  // uniform across the block
+#pragma unroll
+  for (int q = 0; q < NTO; ++q) dft<R, T, false>(w[q]);  // forward pass 1 (NS = 1): outputs at 8 j + r
+  __syncthreads();  // every thread has read its inverse-pass-3 inputs
+#pragma unroll
+  for (int q = 0; q < NTO; ++q)
+#pragma unroll
+    for (int r = 0; r < R; ++r) buf[q * TILE + sw<T, LINES>(R * j + r, line)] = w[q][r];
+  __syncthreads();
+  stockham_pass<T, N, RM, R, LINES, NTO, NT, false, N, true>(buf, tw2, tid);
+  stockham_pass<T, N, R, R * RM, LINES, NTO, NT, false, N, true>(buf, tw3, tid);
+
+  // ---- split W: into S of rows a and b (standard), or into U and V of each row (adjoint)
+#pragma unroll
+  for (int idx = tid; idx < NTO * LINES * (H / 2); idx += NT) {
+    const int t = idx % (H / 2), rest = idx / (H / 2);
+    const int rw = rest % LINES, q = rest / LINES;
+    const c2<T>* wb = buf + q * TILE;
+    c2<T> s0[2], s1[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int k = 2 * t + e;
+      if (k == 0) {
+        const c2<T> w0 = wb[sw<T, LINES>(0, rw)], wh = wb[sw<T, LINES>(H, rw)];
+        s0[0] = mk<T>(w0.x, wh.x);
+        s1[0] = mk<T>(w0.y, wh.y);
+      } else {
+        const c2<T> A = wb[sw<T, LINES>(k, rw)];
+        const c2<T> B = cconj<T>(wb[sw<T, LINES>(N - k, rw)]);
+        s0[e] = cscale<T>(cadd<T>(A, B), T(0.5));
+        const c2<T> d = csub<T>(A, B);
+        s1[e] = mk<T>(T(0.5) * d.y, T(-0.5) * d.x);  // (A - B) / 2i
+      }
+    }
+    if constexpr (ADJ) {
+      st2<T>(spec(a.s) + (q * LINES + rw) * H + 2 * t, s0);
+      st2<T>(spec(a.v) + (q * LINES + rw) * H + 2 * t, s1);
+    } else {
+      st2<T>(spec(a.s) + rw * H + 2 * t, s0);
+      st2<T>(spec(a.s) + (LINES + rw) * H + 2 * t, s1);
+    }
   }
 }
 
