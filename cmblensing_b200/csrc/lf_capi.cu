@@ -534,6 +534,27 @@ cudaError_t run_lens(int N, int C, bool adj, const StageArgs& a, int B, int nste
   }
 }
 
+// phi (a map, or its rfft2) to the five packed derivative spectra: row transform of a map into ``spec``, then
+// the column transforms.  While one map's column tiles leave SMs idle, the three inverse transforms go to blocks
+// of their own (phi precompute with p planes of one map: 64^2 29.7 -> 18.6 us, 128^2 34.8 -> 24.9 us).
+template <int N, typename PK>
+cudaError_t run_phi_spectra(const void* phi, int basis, int B, double2* spec, PK* packed, const double2* tw64,
+                            double kbase, cudaStream_t st) {
+  constexpr int LINES = 8, H = N / 2;
+  constexpr int NT = Geo<double>::nt(N), CLINES = phi_cols_lines(N), NTC = phi_cols_threads(N);
+  const size_t smem_row = sizeof(double2) * (N + LINES * H) + 16;  // + the table's mbarrier
+  const size_t smem_col = sizeof(double2) * (N + CLINES * N) + 16;
+  const int ctiles = (H + 1 + CLINES - 1) / CLINES;
+  const dim3 grid(ctiles, B, (long)ctiles * B * 3 <= 148 ? 3 : 1);
+  if (basis == LF_PHI_FOURIER)
+    return launch<k_phi_cols<N, CLINES, NTC, PK, false>>(grid, NTC, smem_col, st, reinterpret_cast<const double2*>(phi),
+                                                        packed, tw64, kbase);
+  cudaError_t e = launch<k_phi_rows_r2c<N, LINES, NT>>(dim3(N / LINES, B), NT, smem_row, st,
+                                                       reinterpret_cast<const double*>(phi), spec, tw64);
+  if (e != cudaSuccess) return e;
+  return launch<k_phi_cols<N, CLINES, NTC, PK, true>>(grid, NTC, smem_col, st, (const double2*)spec, packed, tw64, kbase);
+}
+
 template <typename TO, int N>
 cudaError_t run_phi_n(const void* phi, int basis, int B, TO* planes, int* min_det, void* ws, const double2* tw64,
                       double kbase, cudaStream_t st) {
@@ -543,21 +564,7 @@ cudaError_t run_phi_n(const void* phi, int basis, int B, TO* planes, int* min_de
   double2* spec = reinterpret_cast<double2*>(ws);            // [B][N][H+1]
   double2* packed = spec + (size_t)B * N * (H + 1);          // [B][5][N][H]
   const size_t smem_row = sizeof(double2) * (N + LINES * H) + 16;  // + the table's mbarrier
-  const size_t smem_col = sizeof(double2) * (N + LINES * N) + 16;  // + the table's mbarrier
-  const int ctiles = (H + 1 + LINES - 1) / LINES;
-  cudaError_t e;
-  if (basis == LF_PHI_MAP) {
-    e = launch<k_phi_rows_r2c<N, LINES, NT>>(dim3(N / LINES, B), NT, smem_row, st,
-                                             reinterpret_cast<const double*>(phi), spec, tw64);
-    if (e != cudaSuccess) return e;
-    e = launch<k_phi_cols_fwd<N, LINES, NT>>(dim3(ctiles, B), NT, smem_col, st, spec, tw64);
-    if (e != cudaSuccess) return e;
-  } else {
-    e = cudaMemcpyAsync(spec, phi, sizeof(double2) * (size_t)B * N * (H + 1), cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return e;
-  }
-  e = launch<k_phi_cols_deriv<N, LINES, NT>>(dim3(ctiles, B), NT, smem_col, st, (const double2*)spec, packed,
-                                             (const double2*)tw64, kbase);
+  cudaError_t e = run_phi_spectra<N>(phi, basis, B, spec, packed, tw64, kbase, st);
   if (e != cudaSuccess) return e;
   e = launch<k_phi_rows_c2r<TO, N, LINES, NT>>(dim3(N / LINES, B * 5), NT, smem_row, st, (const double2*)packed,
                                                planes, (const double2*)tw64);
@@ -575,30 +582,15 @@ cudaError_t run_phi_n(const void* phi, int basis, int B, TO* planes, int* min_de
 template <int N>
 cudaError_t run_phi_pp_n(const void* phi, int basis, int B, float* planes, float* pp, int K, int* min_det, void* ws,
                          const double2* tw64, double kbase, cudaStream_t st) {
-  constexpr int LINES = 8, PL = 2;
-  constexpr int NT = Geo<double>::nt(N);
+  constexpr int PL = 2;
   constexpr int H = N / 2;
   double2* spec = reinterpret_cast<double2*>(ws);
   double2* packed = spec + (size_t)B * N * (H + 1);
-  const size_t smem_row = sizeof(double2) * (N + LINES * H) + 16;
-  const size_t smem_col = sizeof(double2) * (N + LINES * N) + 16;
   const size_t smem_pp = sizeof(double2) * (N + 5 * PL * H) + 16;
-  const int ctiles = (H + 1 + LINES - 1) / LINES;
-  cudaError_t e;
-  if (basis == LF_PHI_MAP) {
-    e = launch<k_phi_rows_r2c<N, LINES, NT>>(dim3(N / LINES, B), NT, smem_row, st,
-                                             reinterpret_cast<const double*>(phi), spec, tw64);
-    if (e != cudaSuccess) return e;
-    e = launch<k_phi_cols_fwd<N, LINES, NT>>(dim3(ctiles, B), NT, smem_col, st, spec, tw64);
-    if (e != cudaSuccess) return e;
-  } else {
-    e = cudaMemcpyAsync(spec, phi, sizeof(double2) * (size_t)B * N * (H + 1), cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return e;
-  }
   constexpr int NTP = pp_threads(N);
+  cudaError_t e;
   if (planes) {  // derivative planes requested too: float64 spectra, so they equal lf_phi_precompute's
-    e = launch<k_phi_cols_deriv<N, LINES, NT>>(dim3(ctiles, B), NT, smem_col, st, (const double2*)spec, packed,
-                                               (const double2*)tw64, kbase);
+    e = run_phi_spectra<N>(phi, basis, B, spec, packed, tw64, kbase, st);
     if (e != cudaSuccess) return e;
     return launch<k_phi_rows_c2r_pp<N, PL, NTP>>(dim3(N / PL, B), NTP, smem_pp, st, (const double2*)packed, planes,
                                                  pp, K, min_det, (const double2*)tw64);
@@ -606,8 +598,7 @@ cudaError_t run_phi_pp_n(const void* phi, int basis, int B, float* planes, float
   // p planes only: the five derivative spectra cross HBM as float32 (the p planes are float32; every
   // transform stays float64): 40 N^2 bytes per map less, phi precompute 1.152 -> 1.078 ms per 64 maps
   float2* packed32 = reinterpret_cast<float2*>(packed);
-  e = launch<k_phi_cols_deriv<N, LINES, NT, float2>>(dim3(ctiles, B), NT, smem_col, st, (const double2*)spec,
-                                                     packed32, (const double2*)tw64, kbase);
+  e = run_phi_spectra<N>(phi, basis, B, spec, packed32, tw64, kbase, st);
   if (e != cudaSuccess) return e;
   return launch<k_phi_rows_c2r_pp<N, PL, NTP, float2>>(dim3(N / PL, B), NTP, smem_pp, st, (const float2*)packed32,
                                                        planes, pp, K, min_det, (const double2*)tw64);

@@ -517,7 +517,7 @@ __device__ __forceinline__ void cl_integrate(const ClusterArgs& a, long cmap) {
   constexpr int E = G::E, TP = G::TP;
   constexpr int TW = cl_tw_size(N, E);
   constexpr long P = (long)N * N;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   c2<T>* data = reinterpret_cast<c2<T>*>(smem_raw);
   c2<T>* tw = data + S::kElems;
   uint64_t* mbar = reinterpret_cast<uint64_t*>(tw + TW);  // [0] the table, [1], [2] the landing areas

@@ -79,6 +79,17 @@ __device__ __forceinline__ float2 f2_fma(float2 a, float2 b, float2 c) {
         "l"(*reinterpret_cast<uint64_t*>(&c)));
   return *reinterpret_cast<float2*>(&r);
 }
+__device__ __forceinline__ float2 f2_mul(float2 a, float2 b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)));
+  return *reinterpret_cast<float2*>(&r);
+}
+// the hardware's approximate reciprocal (about one unit in the last place)
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 // a + s u for a real s
 template <typename T> LF_HD c2<T> caxpy(T s, c2<T> u, c2<T> a) {
 #ifdef __CUDA_ARCH__

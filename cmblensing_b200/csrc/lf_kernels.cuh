@@ -1224,62 +1224,118 @@ __global__ void __launch_bounds__(NT) k_phi_cols_fwd(double2* __restrict__ arr, 
 //   G0 = IFFT_col(F):           phi_y = i KY G0,  phi_yy = -KY^2 G0
 //   G1 = IFFT_col(i KX F):      phi_x = G1,       phi_xy = i KY G1
 //   G2 = IFFT_col(-KX^2 F):     phi_xx = G2
-// (the 1/N^2 of irfft2 folded into the column multiplier).  ``spec`` is the
-// unpacked rfft2 of phi; ``packed`` is [B][5][N][N/2] complex.
-template <int N, int LINES, int NT, typename PK = double2>
-__global__ void __launch_bounds__(NT) k_phi_cols_deriv(const double2* __restrict__ spec, PK* __restrict__ packed,
-                                                        const double2* __restrict__ twN, double kbase) {
+// (the 1/N^2 of irfft2 folded into the column multiplier).  ``in`` is the row
+// transform of phi, FWD (its forward column transform is the first step here),
+// or the rfft2 of phi; ``packed`` is [B][5][N][N/2] complex.
+// The spectrum stays in registers: the forward transform's last pass leaves a
+// thread the inputs of the inverse transforms' first pass, and the last passes
+// write straight to global memory.  (A forward pass over memory, then three
+// loads, multiplies, transforms and stores of the tile through shared memory,
+// moved 48 N^2 bytes more per map: the two kernels took 338 us for 64 maps of 512^2 and 108 us for 48 of
+// 256^2, this one 231 and 43 us.)  Latency of the transforms bounds it (float64 pipe 28% busy, 16 warps per
+// SM, 0.3 of the bandwidth).  grid: x = column tile, y = map, z = 1 or
+// 3: the three transforms one after the other, or each in its own block, which
+// repeats the forward transform but is quicker while SMs are idle.
+// Radices 8 x (N / 64) x 8, one radix-8 butterfly per thread: with radix 16 in a thread's hands the float64
+// spectrum beside the transform needed 255 registers and spilled.
+__host__ __device__ constexpr int phi_cols_lines(int n) { return n == 1024 ? 4 : 8; }
+__host__ __device__ constexpr int phi_cols_threads(int n) { return n / 8 * phi_cols_lines(n); }
+
+template <int N, int LINES, int NT, typename PK, bool FWD>
+__global__ void __launch_bounds__(NT, NT * 128 <= 65536 ? 65536 / (NT * 128) : 1) k_phi_cols(const double2* __restrict__ in, PK* __restrict__ packed,
+                                                 const double2* __restrict__ twN, double kbase) {
+  using T = double;
   using S = decltype(PK::x);  // storage precision of the packed derivative spectra
-  constexpr int H = N / 2;
+  constexpr int H = N / 2, RL = 8, RM = N / 64;  // outer and middle radices
+  using GL = SpGeom<N, RL, LINES, NT>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* tw = reinterpret_cast<double2*>(smem_raw);
   double2* buf = tw + N;
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(buf + LINES * N);
   const int tid = threadIdx.x;
   const int c0 = blockIdx.x * LINES;
-  const long map = blockIdx.y;
-  const double2* a = spec + map * (long)N * (H + 1);
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(buf + LINES * N);
+  const long map = gridDim.y - 1 - blockIdx.y;  // in reverse: the last maps of the row transform are still in L2
+  const double2* a = in + map * (long)N * (H + 1);
   table_copy<N>(tw, twN, mbar, tid);
+  auto src = [=](int m, int line) { return c0 + line <= H ? a[(long)m * (H + 1) + c0 + line] : make_double2(0.0, 0.0); };
+  auto smem = [=](int m, int line) { return buf[sw<T, LINES>(m, line)]; };
+  double2 x[GL::PER][RL];
+  if constexpr (FWD) {
+    sp_read<T, N, RL, 1, LINES, NT, false, N, false>(x, src, tw, tid);
+    sp_write<T, N, RL, 1, LINES, NT>(buf, x, tid);
+    __syncthreads();
+    table_wait(mbar);
+    if constexpr (RM > 1) {
+      double2 v[SpGeom<N, RM, LINES, NT>::PER][RM];
+      sp_read<T, N, RM, RL, LINES, NT, false, N, false>(v, smem, tw, tid);
+      __syncthreads();
+      sp_write<T, N, RM, RL, LINES, NT>(buf, v, tid);
+      __syncthreads();
+    }
+    sp_read<T, N, RL, N / RL, LINES, NT, false, N, false>(x, smem, tw, tid);
+  } else {
+    auto load = [=](int m, int line, double2) { return src(m, line); };
+    sp_apply<T, N, RL, N / RL, LINES, NT>(x, load, tid);
+    __syncthreads();
+    table_wait(mbar);
+  }
   const double scale = 1.0 / (double(N) * double(N));
-  // (G, output j, KY power): KY power 0 = G itself, 1 = i KY G, 2 = -KY^2 G
-  constexpr int kOut[3][2][2] = {{{1, 1}, {4, 2}}, {{0, 0}, {3, 1}}, {{2, 0}, {-1, 0}}};
+  const int g_lo = gridDim.z == 3 ? blockIdx.z : 0, g_hi = gridDim.z == 3 ? blockIdx.z + 1 : 3;
 #pragma unroll 1
-  for (int g = 0; g < 3; ++g) {
-    load_cols<double, N, LINES, NT>(buf, a, H + 1, c0, H + 1, tid);
-    __syncthreads();
-    for (int idx = tid; idx < N * LINES; idx += NT) {
-      const int m = idx / LINES, line = idx % LINES;
+  for (int g = g_lo; g < g_hi; ++g) {
+    double2 y[GL::PER][RL];
+#pragma unroll
+    for (int i = 0; i < GL::PER; ++i)
+#pragma unroll
+      for (int r = 0; r < RL; ++r) y[i][r] = x[i][r];
+    auto mul = [=](int m, int, double2 v) {
       const double kx = kbase * double(m < N / 2 ? m : m - N);
-      const double2 v = buf[sw<double, LINES>(m, line)];
-      double2 r;
-      if (g == 0) r = make_double2(scale * v.x, scale * v.y);
-      else if (g == 1) r = make_double2(-kx * v.y * scale, kx * v.x * scale);
-      else r = make_double2(-kx * kx * scale * v.x, -kx * kx * scale * v.y);
-      buf[sw<double, LINES>(m, line)] = r;
-    }
+      if (g == 0) return make_double2(scale * v.x, scale * v.y);
+      if (g == 1) return make_double2(-kx * v.y * scale, kx * v.x * scale);
+      return make_double2(-kx * kx * scale * v.x, -kx * kx * scale * v.y);
+    };
+    sp_apply<T, N, RL, N / RL, LINES, NT>(y, mul, tid);
+#pragma unroll
+    for (int i = 0; i < GL::PER; ++i)
+      if (GL::TOT % NT == 0 || tid + i * NT < GL::TOT) dft<RL, T, true>(y[i]);
+    __syncthreads();  // the tile's last readers (the forward transform's, or the previous g's) are done
+    sp_write<T, N, RL, 1, LINES, NT>(buf, y, tid);
     __syncthreads();
-    if (g == 0) table_wait(mbar);
-    fft_tiles<double, N, LINES, 1, NT, true, N>(buf, tw, tid);
-    for (int o = 0; o < 2; ++o) {
-      const int j = kOut[g][o][0], pw = kOut[g][o][1];
-      if (j < 0) continue;
-      PK* out = packed + (map * 5 + j) * (long)N * H;
-      for (int idx = tid; idx < N * LINES; idx += NT) {
-        const int m = idx / LINES, line = idx % LINES;
-        const int col = c0 + line;
-        if (col > H) continue;
-        const double ky = (col == H) ? -kbase * double(H) : kbase * double(col);
-        const double2 G = buf[sw<double, LINES>(m, line)];
-        double2 v;
-        if (pw == 0) v = G;
-        else if (pw == 1) v = make_double2(-ky * G.y, ky * G.x);
-        else v = make_double2(-ky * ky * G.x, -ky * ky * G.y);
-        if (col == 0) reinterpret_cast<S*>(out + (long)m * H)[0] = S(v.x);
-        else if (col == H) reinterpret_cast<S*>(out + (long)m * H)[1] = S(v.x);
-        else out[(long)m * H + col] = PK{S(v.x), S(v.y)};
-      }
+    if constexpr (RM > 1) {
+      double2 v[SpGeom<N, RM, LINES, NT>::PER][RM];
+      sp_read<T, N, RM, RL, LINES, NT, true, N, false>(v, smem, tw, tid);
+      __syncthreads();
+      sp_write<T, N, RM, RL, LINES, NT>(buf, v, tid);
+      __syncthreads();
     }
-    __syncthreads();
+    sp_read<T, N, RL, N / RL, LINES, NT, true, N, false>(y, smem, tw, tid);
+    // (output j, KY power) of G0, G1, G2: power 0 = G itself, 1 = i KY G, 2 = -KY^2 G
+    auto put = [=](int j, int pw, int m, int line, double2 G) {
+      const int col = c0 + line;
+      if (col > H) return;
+      const double ky = (col == H) ? -kbase * double(H) : kbase * double(col);
+      const double2 o = pw == 0   ? G
+                        : pw == 1 ? make_double2(-ky * G.y, ky * G.x)
+                                  : make_double2(-ky * ky * G.x, -ky * ky * G.y);
+      PK* row = packed + ((map * 5 + j) * (long)N + m) * H;
+      if (col == 0) reinterpret_cast<S*>(row)[0] = S(o.x);
+      else if (col == H) reinterpret_cast<S*>(row)[1] = S(o.x);
+      else row[col] = PK{S(o.x), S(o.y)};
+    };
+    sp_emit<T, N, RL, N / RL, LINES, NT>(
+        y,
+        [=](int m, int line, double2 G) {
+          if (g == 0) {
+            put(1, 1, m, line, G);
+            put(4, 2, m, line, G);
+          } else if (g == 1) {
+            put(0, 0, m, line, G);
+            put(3, 1, m, line, G);
+          } else {
+            put(2, 0, m, line, G);
+          }
+        },
+        tid);
   }
 }
 
@@ -1313,6 +1369,19 @@ __device__ __forceinline__ int ordered_int(float f) {
   return i >= 0 ? i : i ^ 0x7fffffff;
 }
 
+// Minimum over t in [0, 1] of det(I + t H) = 1 + t l + t^2 q, l = A + C, q = A C - B^2: at t = 1, or at the
+// parabola's vertex t = -l / 2q where that lies inside, i.e. q > 0 and 0 < -l < 2 q.  (A real H has l^2 >= 4 q,
+// so that takes q > 1: the division is for the strongest distortions alone.)
+__device__ __forceinline__ double min_det_01(double A, double B, double C) {
+  const double q = A * C - B * B, l = A + C;
+  double d = 1.0 + l + q;
+  if (q > 0.0 && l < 0.0 && -l < 2.0 * q) {
+    const double ts = -l / (2.0 * q);
+    d = fmin(d, 1.0 + ts * l + ts * ts * q);
+  }
+  return d;
+}
+
 template <typename T>
 __global__ void k_min_det(const T* __restrict__ planes, long P, int* __restrict__ out) {
   const long map = blockIdx.y;
@@ -1321,13 +1390,7 @@ __global__ void k_min_det(const T* __restrict__ planes, long P, int* __restrict_
   const T* pyy = pxy + P;
   double best = 1.0;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < P; i += (long)gridDim.x * blockDim.x) {
-    const double A = pxx[i], B = pxy[i], Cc = pyy[i];
-    const double q = A * Cc - B * B, l = A + Cc;
-    double d = 1.0 + l + q;  // t = 1
-    if (q > 0.0) {
-      const double ts = -l / (2.0 * q);
-      if (ts > 0.0 && ts < 1.0) d = fmin(d, 1.0 + ts * l + ts * ts * q);
-    }
+    const double d = min_det_01(pxx[i], pxy[i], pyy[i]);
     best = fmin(best, d);
   }
   for (int o = 16; o > 0; o >>= 1) best = fmin(best, __shfl_xor_sync(0xffffffffu, best, o));
@@ -1397,49 +1460,47 @@ __global__ void __launch_bounds__(NT, N == 1024 ? 2 : 4) k_phi_rows_c2r_pp(const
             make_float4(float(d[j][0]), float(d[j][1]), float(d[j][2]), float(d[j][3]));
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {  // min over t in [0, 1] of det(I + t H) = 1 + t l + t^2 qd
-      const double A = d[2][q], B = d[3][q], Cc = d[4][q];
-      const double qd = A * Cc - B * B, l = A + Cc;
-      double dm = 1.0 + l + qd;
-      if (qd > 0.0) {
-        const double ts = -l / (2.0 * qd);
-        if (ts > 0.0 && ts < 1.0) dm = fmin(dm, 1.0 + ts * l + ts * ts * qd);
-      }
-      best = fmin(best, dm);
-    }
+    for (int q = 0; q < 4; ++q) best = fmin(best, min_det_01(d[2][q], d[3][q], d[4][q]));
     float* out = pp + map * (long)K * 2 * P + o;
     // p = M(t)^-1 grad phi through the adjugate of the symmetric 2x2 M = I + t H (H = grad grad phi):
     //   p_x = (phi_x + t (H_yy phi_x - H_xy phi_y)) / D,  p_y = (phi_y + t (H_xx phi_y - H_xy phi_x)) / D,
     //   D = det M = 1 + t (H_xx + H_yy) + t^2 (H_xx H_yy - H_xy^2).
     // The time-independent coefficients are formed once per pixel in float64; each time then costs two
-    // FMAs for D, one reciprocal and four FMA/multiplies in float32 (the RK4 right-hand side that reads
-    // the planes is float32).  The reference's det + 1e-12 (lense_flow.py:408-411) is below float32
-    // resolution for D >= 0.2 and is not added.
-    float gx[4], gy[4], bx[4], by[4], lt[4], qt[4];
+    // FMAs for D, a reciprocal and four FMA/multiplies in float32 (the RK4 right-hand side that reads the
+    // planes is float32), on pixel pairs in packed arithmetic.  The reference's det + 1e-12
+    // (lense_flow.py:408-411) is below float32 resolution for D >= 0.2 and is not added.  (Scalar, with
+    // correctly rounded reciprocals, the loop was a third of this pass's 684 instructions per pixel.)
+    float2 gx[2], gy[2], bx[2], by[2], lt[2], qt[2];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const double A = d[2][q], Bx = d[3][q], Cc = d[4][q];
-      gx[q] = float(d[0][q]);
-      gy[q] = float(d[1][q]);
-      bx[q] = float(Cc * d[0][q] - Bx * d[1][q]);
-      by[q] = float(A * d[1][q] - Bx * d[0][q]);
-      lt[q] = float(A + Cc);
-      qt[q] = float(A * Cc - Bx * Bx);
+    for (int q = 0; q < 2; ++q) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int i = 2 * q + u;
+        const double A = d[2][i], Bx = d[3][i], Cc = d[4][i];
+        float* const o6[6] = {&gx[q].x, &gy[q].x, &bx[q].x, &by[q].x, &lt[q].x, &qt[q].x};
+        const double v6[6] = {d[0][i],   d[1][i], Cc * d[0][i] - Bx * d[1][i], A * d[1][i] - Bx * d[0][i],
+                              A + Cc, A * Cc - Bx * Bx};
+#pragma unroll
+        for (int c = 0; c < 6; ++c) o6[c][u] = float(v6[c]);
+      }
     }
+    const float2 one = make_float2(1.0f, 1.0f);
 #pragma unroll 1
     for (int k = 0; k < K; ++k) {
       const float t = float(double(k) * inv2n);
-      float ox[4], oy[4];
+      const float2 tt = make_float2(t, t);
+      float2 ox[2], oy[2];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float r = __frcp_rn(fmaf(t, fmaf(t, qt[q], lt[q]), 1.0f));
-        ox[q] = fmaf(t, bx[q], gx[q]) * r;
-        oy[q] = fmaf(t, by[q], gy[q]) * r;
+      for (int q = 0; q < 2; ++q) {
+        const float2 D = f2_fma(tt, f2_fma(tt, qt[q], lt[q]), one);
+        // 1 / D: the hardware approximation and one Newton step, r + r (1 - D r)
+        float2 r = make_float2(rcp_approx(D.x), rcp_approx(D.y));
+        r = f2_fma(r, f2_fma(make_float2(-D.x, -D.y), r, one), r);
+        ox[q] = f2_mul(f2_fma(tt, bx[q], gx[q]), r);
+        oy[q] = f2_mul(f2_fma(tt, by[q], gy[q]), r);
       }
-      *reinterpret_cast<float4*>(out + (2 * k) * P) =
-          make_float4(float(ox[0]), float(ox[1]), float(ox[2]), float(ox[3]));
-      *reinterpret_cast<float4*>(out + (2 * k + 1) * P) =
-          make_float4(float(oy[0]), float(oy[1]), float(oy[2]), float(oy[3]));
+      *reinterpret_cast<float4*>(out + (2 * k) * P) = make_float4(ox[0].x, ox[0].y, ox[1].x, ox[1].y);
+      *reinterpret_cast<float4*>(out + (2 * k + 1) * P) = make_float4(oy[0].x, oy[0].y, oy[1].x, oy[1].y);
     }
   }
   if (min_det) {
