@@ -348,13 +348,28 @@ def chunk_schedule(batch, chunks=8, chunk_sizes=None):
     return chunk_sizes
 
 
+DEFAULT_CHUNKS = 8
+
+
+def default_chunks(call_bytes):
+    """Chunks of a HostPipeline call that copies ``call_bytes`` to the device, up to DEFAULT_CHUNKS.
+
+    More chunks hide more of the first upload and the last download, fewer cost less compute per map and
+    fewer launches; the best number grows with about the square root of the bytes.  Measured with 8 chunks
+    and with this many, us per waiting (queued) call: 12 QU maps of 512^2 (50 MB) 2,339 (2,062) and 2,046
+    (1,478), 24 QU of 256^2 (25 MB) 1,058 (836) and 988 (659), 16 TQU of 128^2 (5 MB) 633 (553) and 374
+    (229), 3 T of 64^2 293 (256) and 166 (133); at 126 MB and above 8 is the best or within 3% of it."""
+    return max(1, min(DEFAULT_CHUNKS, round(0.7 * (call_bytes / 1e6) ** 0.5)))
+
+
 class HostPipeline:
     """The reference-facing call with host buffers, for a fixed batch, pipelined.
 
     Each call copies f [B,C,N,N] and phi [B,N,N] (pinned host memory) to the
     device, computes the phi derivative planes (with the magnification check),
     lenses, and copies the result back into a pinned host buffer.  The batch
-    is split into ``chunks`` that move through ``slots`` sets of device
+    is split into ``chunks`` (the default takes fewer for small calls, see
+    ``default_chunks``; any other number is taken as given) that move through ``slots`` sets of device
     buffers: host-to-device copies on one stream, compute alternating between
     ``compute_streams`` streams, device-to-host copies on another.  A chunk's
     lens is a few dozen short launches; with two compute streams the kernels
@@ -384,21 +399,23 @@ class HostPipeline:
     is known).
     """
 
-    def __init__(self, plan, batch, io_dtype=torch.float64, chunks=8, compute_streams=2, slots=4,
+    def __init__(self, plan, batch, io_dtype=torch.float64, chunks=DEFAULT_CHUNKS, compute_streams=2, slots=4,
                  use_graphs=True, chunk_sizes=None):
         self.plan = plan
         N, C = plan.nside, plan.ncomp
         dev = plan.device
         self.batch = batch
+        self.io_dtype = io_dtype
+        if chunk_sizes is None and chunks == DEFAULT_CHUNKS:
+            chunks = default_chunks(self.h2d_bytes())
         chunk_sizes = chunk_schedule(batch, chunks, chunk_sizes)
         self.sizes = chunk_sizes
         self.offsets = [sum(chunk_sizes[:i]) for i in range(len(chunk_sizes))]
         self.chunks = len(chunk_sizes)
         self.cb = max(chunk_sizes, default=1)  # device buffers hold the largest chunk
         cb = self.cb
-        self.io_dtype = io_dtype
         self.nslots = max(2, int(slots))
-        ns = self.nslots
+        ns = min(self.nslots, max(1, self.chunks))  # a call's chunk i uses slot i % nslots
         self.d_f = [torch.empty((cb, C, N, N), dtype=io_dtype, device=dev) for _ in range(ns)]
         self.d_out = [torch.empty((cb, C, N, N), dtype=io_dtype, device=dev) for _ in range(ns)]
         self.d_phi = [torch.empty((cb, N, N), dtype=torch.float64, device=dev) for _ in range(ns)]
@@ -493,7 +510,7 @@ class HostPipeline:
         if self.use_pp and n not in self.pp:
             N = plan.nside
             self.pp[n] = [torch.empty((self.cb, 2 * int(n) + 1, 2, N, N), dtype=torch.float32, device=plan.device)
-                          for _ in range(self.nslots)]
+                          for _ in range(len(self.d_f))]
         cur = torch.cuda.current_stream(plan.device)
         streams = [self.s_in, self.s_out] + self.s_cmp
         for st in streams:

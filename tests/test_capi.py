@@ -105,3 +105,11 @@ def test_host_pipeline_chunk_schedule():
     for bad in ([1, 2, 4], [0, 4, 4], [9, -1]):
         with pytest.raises(ValueError):
             chunk_schedule(8, 4, bad)
+
+
+def test_host_pipeline_default_chunks():
+    """The default chunk count: one for the smallest calls, monotonic in the bytes, at most eight."""
+    from cmblensing_b200.engine import DEFAULT_CHUNKS, default_chunks
+    assert default_chunks(0) == default_chunks(1e5) == 1
+    counts = [default_chunks(b) for b in (1e6, 5e6, 2e7, 5e7, 1e8, 1.3e8, 4e8, 1e10)]
+    assert counts == sorted(counts) and counts[-3:] == [DEFAULT_CHUNKS] * 3
