@@ -269,21 +269,22 @@ cudaError_t launch(dim3 grid, int nt, size_t smem, cudaStream_t st, Args... args
   return launch_k<Kernel>(LF_KIND_PHI, grid, nt, smem, st, args...);
 }
 
-// One column pass over `planes` packed row-spectrum planes.  FP32 512: the
-// two-pass plan 16 x 32 in 256-thread blocks; otherwise the pass-table plan.
+// One column pass over `planes` packed row-spectrum planes.  FP32 512 and 1024: the two-pass plan, one radix-32
+// butterfly per thread and two blocks of 256 threads per SM; otherwise the pass-table plan.
 template <typename T, int N>
 cudaError_t launch_col(int planes, cudaStream_t st, const StageArgs& a) {
-  constexpr int LINES = Geo<T>::LINES;
-  const dim3 grid(N / 2 / LINES, planes);
   if constexpr (std::is_same<T, float>::value && col2_plan(N)) {
-    // 16-line tiles (128-byte row segments), 256 threads (one radix-32 butterfly each), 2 blocks per SM
-    constexpr int NT2 = 256;
-    const size_t smem = sizeof(c2<T>) * (col_tw_entries(N, true) + LINES * N) + 16;  // + the table's mbarrier
-    return launch_k<k_col<T, N, LINES, NT2, 2, true>>(LF_KIND_COL, grid, NT2, smem, st, a);
+    // 512: 16-line tiles (128-byte row segments).  1024: 8 lines, so that two tiles fit an SM; one lens of 3 TQU
+    // maps (n = 7) 2,346 us with the three-pass plan (one block of 1,024 threads), 2,229 with 16-line tiles in
+    // the two-pass plan (one block), 2,171 with 8; 16 maps (n = 5) 7,865 and 7,545; one T map 621, 566 and 587.
+    constexpr int CL = N == 512 ? 16 : 8, NT2 = 256;
+    const size_t smem = sizeof(c2<T>) * (col_tw_entries(N, true) + CL * N) + 16;  // + the table's mbarrier
+    return launch_k<k_col<T, N, CL, NT2, 2, true>>(LF_KIND_COL, dim3(N / 2 / CL, planes), NT2, smem, st, a);
   } else {
+    constexpr int LINES = Geo<T>::LINES;
     constexpr int NT = Geo<T>::nt(N);
     const size_t smem = sizeof(c2<T>) * (col_tw_entries(N) + LINES * N) + 16;  // + the table's mbarrier
-    return launch_k<k_col<T, N, LINES, NT, Geo<T>::minb(N)>>(LF_KIND_COL, grid, NT, smem, st, a);
+    return launch_k<k_col<T, N, LINES, NT, Geo<T>::minb(N)>>(LF_KIND_COL, dim3(N / 2 / LINES, planes), NT, smem, st, a);
   }
 }
 
@@ -336,7 +337,13 @@ cudaError_t run_lens_pp(const StageArgs& base, int B, int nsteps, double t0, dou
   const bool use_pdl = (long)B * C * N * N <= (1L << 23);
   PdlScope pdl;
   if (PP && use_pdl) pdl.enable();
-  e = launch_k<k_row<T, N, C, ADJ, true, RL, RNT, false, RMB, PP>>(LF_KIND_ROW, grow, RNT, smem_row, st, a);
+  if constexpr (PP && std::is_same<T, float>::value) {
+    constexpr int PL = 1024 / N, PNT = (N / 8) * PL;
+    e = launch_k<k_row_rows<N, PL, PNT, 6, ADJ, true>>(LF_KIND_ROW, dim3(N / (2 * PL), B * C), PNT,
+                                                       row_rows_smem_bytes<N, PL>(true), st, a);
+  } else {
+    e = launch_k<k_row<T, N, C, ADJ, true, RL, RNT, false, RMB>>(LF_KIND_ROW, grow, RNT, smem_row, st, a);
+  }
   if (e != cudaSuccess) return e;
   if (use_pdl) pdl.enable();
   for (int i = 0; i < nsteps; ++i) {
@@ -370,10 +377,10 @@ cudaError_t run_lens_pp(const StageArgs& base, int B, int nsteps, double t0, dou
       } else if constexpr (PP && std::is_same<T, float>::value) {
         // other shapes with p planes: row pairs of one component, 128 threads, five blocks per SM
         constexpr int PL = 1024 / N, PNT = (N / 8) * PL;
-        e = launch_k<k_row_rows<N, PL, PNT, 5, ADJ>>(LF_KIND_ROW, dim3(N / (2 * PL), B * C), PNT,
-                                                     row_rows_smem_bytes<N, PL>(), st, a);
+        e = launch_k<k_row_rows<N, PL, PNT, 5, ADJ, false>>(LF_KIND_ROW, dim3(N / (2 * PL), B * C), PNT,
+                                                            row_rows_smem_bytes<N, PL>(false), st, a);
       } else {
-        e = launch_k<k_row<T, N, C, ADJ, false, RL, RNT, false, RMB, PP>>(LF_KIND_ROW, grow, RNT, smem_row, st, a);
+        e = launch_k<k_row<T, N, C, ADJ, false, RL, RNT, false, RMB>>(LF_KIND_ROW, grow, RNT, smem_row, st, a);
       }
       if (e != cudaSuccess) return e;
     }

@@ -513,13 +513,13 @@ __device__ __forceinline__ void fft_mul_ifft_2p(c2<T>* buf, const c2<T>* twf, co
   sp_emit<T, L, R1, R2, LINES, NT>(a, dst, tid);
 }
 
-// Column table: the two-pass plan 512 = 16 x 32 of the column pass.  Block
-// (R 32, NS 16) of the forward pass 2 at entry 0, block (R 16, NS 32) of the
-// inverse pass 2 after it; lengths without a two-pass column plan have none.
-__host__ __device__ constexpr bool col2_plan(int L) { return L == 512; }
-__host__ __device__ constexpr int col2_r1(int) { return 16; }
+// Column table: the two-pass plans 512 = 16 x 32 and 1024 = 32 x 32 of the column pass.  Block (R2, NS R1) of
+// the forward pass 2 at entry 0, block (R1, NS R2) of the inverse pass 2 after it (the same one for 1024);
+// lengths without a two-pass column plan have none.
+__host__ __device__ constexpr bool col2_plan(int L) { return L == 512 || L == 1024; }
+__host__ __device__ constexpr int col2_r1(int L) { return L / 32; }
 __host__ __device__ constexpr int col2_r2(int) { return 32; }
-__host__ __device__ constexpr int ctw_inv_offset(int L) { return col2_plan(L) ? (col2_r2(L) - 1) * col2_r1(L) : 0; }
+__host__ __device__ constexpr int ctw_inv_offset(int L) { return L == 512 ? (col2_r2(L) - 1) * col2_r1(L) : 0; }
 __host__ __device__ constexpr int ctw_size(int L) {
   return col2_plan(L) ? ctw_inv_offset(L) + (col2_r1(L) - 1) * col2_r2(L) : 0;
 }

@@ -218,7 +218,7 @@ __device__ __forceinline__ bool wait_or_record(uint64_t* mbar, uint32_t parity) 
 
 // ======================================================== column pass
 // Gx = IFFT_col( (i KX / N^2) * FFT_col(S) ) on tiles of LINES columns.
-// grid: x = column tile (N/2/LINES), y = plane.  TWO: the plan N = 16 x 32
+// grid: x = column tile (N/2/LINES), y = plane.  TWO: the plan N = 16 x 32 or 32 x 32
 // (one shared-memory round trip per direction) instead of 8 x 8 x 8.
 template <typename T, int N, int LINES, int NT, int MINB = 1, bool TWO = false>
 __global__ void __launch_bounds__(NT, MINB) k_col(StageArgs a) {
@@ -282,10 +282,8 @@ __global__ void __launch_bounds__(NT, MINB) k_col(StageArgs a) {
 // STAGE0: initialisation (copy the input field, transform the first stage
 // input), no rate.  SAVE (reverse mode): the standard pass also stores
 // d_x y_s and d_y y_s; the adjoint pass stores its next stage input.
-// PP: p at the stage time is read from the precomputed p planes (two loads per
-// pixel) instead of being formed from the five derivative planes.
-template <typename T, int N, int C, bool ADJ, bool STAGE0, int LINES, int NT, bool SAVE = false, int MINB = 1,
-          bool PP = false>
+// p is formed from the five derivative planes; lenses with p planes take the row-pair passes below.
+template <typename T, int N, int C, bool ADJ, bool STAGE0, int LINES, int NT, bool SAVE = false, int MINB = 1>
 __global__ void __launch_bounds__(NT, MINB) k_row(StageArgs a) {
   constexpr int H = N / 2;
   constexpr long P = (long)N * N;
@@ -372,31 +370,17 @@ __global__ void __launch_bounds__(NT, MINB) k_row(StageArgs a) {
     // p at the rate time (standard) and at the next stage time (adjoint)
     T prx[2][2], pry[2][2];
     if (need_phi) {
-      if constexpr (PP) {
-        const T* pp = reinterpret_cast<const T*>(a.pp) + (map * a.pp_k + a.pp_idx) * 2 * P + (long)r0 * N;
-        c2<T> px[2], py[2];
-        ld2<T>(reinterpret_cast<const c2<T>*>(pp) + e0, px);
-        ld2<T>(reinterpret_cast<const c2<T>*>(pp + P) + e0, py);
+      c2<T> fx[2], fy[2], fxx[2], fxy[2], fyy[2];
+      ld2<T>(reinterpret_cast<const c2<T>*>(phi) + e0, fx);
+      ld2<T>(reinterpret_cast<const c2<T>*>(phi + P) + e0, fy);
+      ld2<T>(reinterpret_cast<const c2<T>*>(phi + 2 * P) + e0, fxx);
+      ld2<T>(reinterpret_cast<const c2<T>*>(phi + 3 * P) + e0, fxy);
+      ld2<T>(reinterpret_cast<const c2<T>*>(phi + 4 * P) + e0, fyy);
+      const T tp = ADJ ? tnext : tcur;
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          prx[q][0] = px[q].x;
-          prx[q][1] = px[q].y;
-          pry[q][0] = py[q].x;
-          pry[q][1] = py[q].y;
-        }
-      } else {
-        c2<T> fx[2], fy[2], fxx[2], fxy[2], fyy[2];
-        ld2<T>(reinterpret_cast<const c2<T>*>(phi) + e0, fx);
-        ld2<T>(reinterpret_cast<const c2<T>*>(phi + P) + e0, fy);
-        ld2<T>(reinterpret_cast<const c2<T>*>(phi + 2 * P) + e0, fxx);
-        ld2<T>(reinterpret_cast<const c2<T>*>(phi + 3 * P) + e0, fxy);
-        ld2<T>(reinterpret_cast<const c2<T>*>(phi + 4 * P) + e0, fyy);
-        const T tp = ADJ ? tnext : tcur;
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          p_vector<T>(fx[q].x, fy[q].x, fxx[q].x, fxy[q].x, fyy[q].x, tp, prx[q][0], pry[q][0]);
-          p_vector<T>(fx[q].y, fy[q].y, fxx[q].y, fxy[q].y, fyy[q].y, tp, prx[q][1], pry[q][1]);
-        }
+      for (int q = 0; q < 2; ++q) {
+        p_vector<T>(fx[q].x, fy[q].x, fxx[q].x, fxy[q].x, fyy[q].x, tp, prx[q][0], pry[q][0]);
+        p_vector<T>(fx[q].y, fy[q].y, fxx[q].y, fxy[q].y, fyy[q].y, tp, prx[q][1], pry[q][1]);
       }
     }
 #pragma unroll
@@ -919,11 +903,12 @@ __global__ void __launch_bounds__(NT, MINB) k_row_pair_adj(StageArgs a) {
 __host__ __device__ constexpr int rtw_mid(int n) { return n / 64; }  // radix of the middle pass
 __host__ __device__ constexpr int rtw_size(int n) { return (rtw_mid(n) - 1) * 8 + 7 * (n / 8); }
 
-template <int N, int LINES> constexpr size_t row_rows_smem_bytes() {
-  return sizeof(float2) * (rtw_size(N) + 2 * LINES * N) + sizeof(float) * 4 * LINES * N + 16;
+// INIT: the integration's first launch, which only copies the input field to y0 and transforms it.
+template <int N, int LINES> constexpr size_t row_rows_smem_bytes(bool init) {
+  return sizeof(float2) * (rtw_size(N) + 2 * LINES * N) + (init ? 0 : sizeof(float) * 4 * LINES * N) + 16;
 }
 
-template <int N, int LINES, int NT, int MINB, bool ADJ>
+template <int N, int LINES, int NT, int MINB, bool ADJ, bool INIT>
 __global__ void __launch_bounds__(NT, MINB) k_row_rows(StageArgs a) {
   using T = float;
   constexpr int H = N / 2;
@@ -940,7 +925,7 @@ __global__ void __launch_bounds__(NT, MINB) k_row_rows(StageArgs a) {
   c2<T>* tw = reinterpret_cast<c2<T>*>(smem_raw);
   c2<T>* buf = tw + rtw_size(N);                     // tile q at buf + q * TILE
   T* stg = reinterpret_cast<T*>(buf + 2 * TILE);     // y0, then acc, of the block's rows
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(stg + 2 * RB);  // [0]: staged update operands, [1]: spectra
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(INIT ? stg : stg + 2 * RB);  // [0]: staged update operands, [1]: spectra
   const int tid = threadIdx.x;
   const int r0 = blockIdx.x * 2 * LINES;
   const long plane = blockIdx.y, map = plane / a.ncomp;
@@ -952,21 +937,23 @@ __global__ void __launch_bounds__(NT, MINB) k_row_rows(StageArgs a) {
   if (tid == 0) {
     mbar_init(mbar, 1);
     mbar_init(mbar + 1, 1);
-    mbar_expect_tx(mbar + 1, uint32_t(rtw_size(N) * sizeof(c2<T>) + 4 * LINES * H * sizeof(c2<T>)));
+    mbar_expect_tx(mbar + 1, uint32_t((rtw_size(N) + (INIT ? 0 : 4 * LINES * H)) * sizeof(c2<T>)));
     bulk_g2s(tw, a.twR, rtw_size(N) * sizeof(c2<T>), mbar + 1);
     pdl_wait();  // the other copies read what the previous kernel wrote
-    for (int q = 0; q < 2; ++q) {  // Gx, then S (adjoint: V), of the tile's rows, packed
+    for (int q = 0; q < (INIT ? 0 : 2); ++q) {  // Gx, then S (adjoint: V), of the tile's rows, packed
       bulk_g2s(buf + q * TILE, spec(a.gx) + q * LINES * H, LINES * H * sizeof(c2<T>), mbar + 1);
       bulk_g2s(buf + q * TILE + LINES * H, spec(ADJ ? a.v : a.s) + q * LINES * H, LINES * H * sizeof(c2<T>), mbar + 1);
     }
-    mbar_expect_tx(mbar, uint32_t((with_acc ? 2 : 1) * RB * sizeof(T)));
-    bulk_g2s(stg, reinterpret_cast<const T*>(a.y0) + plane * P + prow0, RB * sizeof(T), mbar);
-    if (with_acc) bulk_g2s(stg + RB, reinterpret_cast<const T*>(a.acc) + plane * P + prow0, RB * sizeof(T), mbar);
+    if constexpr (!INIT) {
+      mbar_expect_tx(mbar, uint32_t((with_acc ? 2 : 1) * RB * sizeof(T)));
+      bulk_g2s(stg, reinterpret_cast<const T*>(a.y0) + plane * P + prow0, RB * sizeof(T), mbar);
+    }
+    if (!INIT && with_acc) bulk_g2s(stg + RB, reinterpret_cast<const T*>(a.acc) + plane * P + prow0, RB * sizeof(T), mbar);
   }
   pdl_wait();  // every thread, before its own global reads and writes
   const int j = tid % NB, line = tid / NB;
   T px[2][R], py[2][R];  // p (adjoint: at the next stage's time) of the thread's pixels, hidden under the transforms
-  {
+  if constexpr (ADJ || !INIT) {
     const T* pq = reinterpret_cast<const T*>(a.pp) + (map * a.pp_k + a.pp_idx) * 2 * P + prow0 + line * N + j;
 #pragma unroll
     for (int q = 0; q < 2; ++q)
@@ -983,99 +970,114 @@ __global__ void __launch_bounds__(NT, MINB) k_row_rows(StageArgs a) {
   // a timed-out wait is recorded and the block goes on, so that every thread meets every barrier below
   wait_or_record(mbar + 1, 0);
 
-  // ------------- load: the packed rows sit in the tiles; all of them are read before Z overwrites them
-  c2<T> gv[2][IT][2], sv[2][IT][2];
+  c2<T> w[2][R];
+  if constexpr (INIT) {
 #pragma unroll
-  for (int q = 0; q < 2; ++q)
+    for (int r = 0; r < R; ++r) {
+      T yn[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const long fo = plane * P + prow0 + (q * LINES + line) * N + j + NB * r;
+        yn[q] = a.in_f64 ? T(reinterpret_cast<const double*>(a.f_in)[fo]) : reinterpret_cast<const float*>(a.f_in)[fo];
+        reinterpret_cast<T*>(a.y0)[fo] = yn[q];
+        if constexpr (ADJ) w[q][r] = mk<T>(px[q][r] * yn[q], py[q][r] * yn[q]);
+      }
+      if constexpr (!ADJ) w[0][r] = mk<T>(yn[0], yn[1]);
+    }
+  } else {
+    // ------------- load: the packed rows sit in the tiles; all of them are read before Z overwrites them
+    c2<T> gv[2][IT][2], sv[2][IT][2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int it = 0; it < IT; ++it) {
+        const int idx = tid + it * NT, t = idx % (H / 2), row = idx / (H / 2);
+        ld2<T>(buf + q * TILE + row * H + 2 * t, gv[q][it]);
+        ld2<T>(buf + q * TILE + LINES * H + row * H + 2 * t, sv[q][it]);
+      }
+    __syncthreads();
 #pragma unroll
     for (int it = 0; it < IT; ++it) {
       const int idx = tid + it * NT, t = idx % (H / 2), row = idx / (H / 2);
-      ld2<T>(buf + q * TILE + row * H + 2 * t, gv[q][it]);
-      ld2<T>(buf + q * TILE + LINES * H + row * H + 2 * t, sv[q][it]);
-    }
-  __syncthreads();
 #pragma unroll
-  for (int it = 0; it < IT; ++it) {
-    const int idx = tid + it * NT, t = idx % (H / 2), row = idx / (H / 2);
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int k = 2 * t + e;
-      const T f = ky_scale * T(k);
-      if constexpr (ADJ) {
-        if (k == 0) {  // real DC and Nyquist bins of each rate; i KY contributes nothing there
-          buf[sw<T, LINES>(0, row)] = mk<T>(gv[0][it][0].x, gv[1][it][0].x);
-          buf[sw<T, LINES>(H, row)] = mk<T>(gv[0][it][0].y, gv[1][it][0].y);
-        } else {
-          const c2<T> k0 = mk<T>(gv[0][it][e].x - f * sv[0][it][e].y, gv[0][it][e].y + f * sv[0][it][e].x);
-          const c2<T> k1 = mk<T>(gv[1][it][e].x - f * sv[1][it][e].y, gv[1][it][e].y + f * sv[1][it][e].x);
-          buf[sw<T, LINES>(k, row)] = mk<T>(k0.x - k1.y, k0.y + k1.x);      // K_a + i K_b
-          buf[sw<T, LINES>(N - k, row)] = mk<T>(k0.x + k1.y, k1.x - k0.y);  // conj(K_a) + i conj(K_b)
-        }
-      } else {
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          c2<T>* z = buf + q * TILE;
-          const c2<T> g = gv[q][it][e], sq = sv[q][it][e];
-          if (k == 0) {
-            z[sw<T, LINES>(0, row)] = mk<T>(g.x, T(0));
-            z[sw<T, LINES>(H, row)] = mk<T>(g.y, T(0));
+      for (int e = 0; e < 2; ++e) {
+        const int k = 2 * t + e;
+        const T f = ky_scale * T(k);
+        if constexpr (ADJ) {
+          if (k == 0) {  // real DC and Nyquist bins of each rate; i KY contributes nothing there
+            buf[sw<T, LINES>(0, row)] = mk<T>(gv[0][it][0].x, gv[1][it][0].x);
+            buf[sw<T, LINES>(H, row)] = mk<T>(gv[0][it][0].y, gv[1][it][0].y);
           } else {
-            z[sw<T, LINES>(k, row)] = mk<T>(g.x - f * sq.x, g.y - f * sq.y);       // DX + i DY, DY = i f S
-            z[sw<T, LINES>(N - k, row)] = mk<T>(g.x + f * sq.x, -g.y - f * sq.y);  // conj(DX) + i conj(DY)
+            const c2<T> k0 = mk<T>(gv[0][it][e].x - f * sv[0][it][e].y, gv[0][it][e].y + f * sv[0][it][e].x);
+            const c2<T> k1 = mk<T>(gv[1][it][e].x - f * sv[1][it][e].y, gv[1][it][e].y + f * sv[1][it][e].x);
+            buf[sw<T, LINES>(k, row)] = mk<T>(k0.x - k1.y, k0.y + k1.x);      // K_a + i K_b
+            buf[sw<T, LINES>(N - k, row)] = mk<T>(k0.x + k1.y, k1.x - k0.y);  // conj(K_a) + i conj(K_b)
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            c2<T>* z = buf + q * TILE;
+            const c2<T> g = gv[q][it][e], sq = sv[q][it][e];
+            if (k == 0) {
+              z[sw<T, LINES>(0, row)] = mk<T>(g.x, T(0));
+              z[sw<T, LINES>(H, row)] = mk<T>(g.y, T(0));
+            } else {
+              z[sw<T, LINES>(k, row)] = mk<T>(g.x - f * sq.x, g.y - f * sq.y);       // DX + i DY, DY = i f S
+              z[sw<T, LINES>(N - k, row)] = mk<T>(g.x + f * sq.x, -g.y - f * sq.y);  // conj(DX) + i conj(DY)
+            }
           }
         }
       }
     }
-  }
-  __syncthreads();
-  stockham_pass<T, N, R, 1, LINES, NTI, NT, true, N, true>(buf, tw, tid);
-  stockham_pass<T, N, RM, R, LINES, NTI, NT, true, N, true>(buf, tw2, tid);
+    __syncthreads();
+    stockham_pass<T, N, R, 1, LINES, NTI, NT, true, N, true>(buf, tw, tid);
+    stockham_pass<T, N, RM, R, LINES, NTI, NT, true, N, true>(buf, tw2, tid);
 
-  // ----------------- inverse pass 3 -> RK4 update -> forward pass 1, in registers
-  c2<T> v[2][R];
+    // ----------------- inverse pass 3 -> RK4 update -> forward pass 1, in registers
+    c2<T> v[2][R];
 #pragma unroll
-  for (int q = 0; q < NTI; ++q)
+    for (int q = 0; q < NTI; ++q)
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[q][r] = buf[q * TILE + sw<T, LINES>(j + r * NB, line)];
+      for (int r = 0; r < R; ++r) v[q][r] = buf[q * TILE + sw<T, LINES>(j + r * NB, line)];
 #pragma unroll
-  for (int r = 1; r < R; ++r) {
-    const c2<T> w = tw3[(r - 1) * NB + j];  // W_N^(r j): NS = N / R
+    for (int r = 1; r < R; ++r) {
+      const c2<T> w = tw3[(r - 1) * NB + j];  // W_N^(r j): NS = N / R
 #pragma unroll
-    for (int q = 0; q < NTI; ++q) v[q][r] = twmul<T, true>(v[q][r], w);
-  }
-#pragma unroll
-  for (int q = 0; q < NTI; ++q) dft<R, T, true>(v[q]);
-  // standard: v[q][r] = dx + i dy at pixel n = j + NB r of row q; adjoint: v[0][r] = (k_a, k_b)
-  if (!wait_or_record(mbar, 0)) return;  // the staged operands: recorded, drained, leave
-  const T hh = T(a.h);
-  c2<T> w[2][R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    T yn[2];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int n = (q * LINES + line) * N + j + NB * r;  // within the block's rows
-      const T k = ADJ ? (q == 0 ? v[0][r].x : v[0][r].y) : px[q][r] * v[q][r].x + py[q][r] * v[q][r].y;
-      const T y0 = stg[n];
-      T* accg = reinterpret_cast<T*>(a.acc) + plane * P + prow0;
-      if (a.stage == 1) {
-        yn[q] = y0 + T(0.5) * hh * k;
-        accg[n] = k;
-      } else if (a.stage < 4) {
-        yn[q] = y0 + (a.stage == 2 ? T(0.5) * hh : hh) * k;
-        accg[n] = stg[RB + n] + T(2) * k;
-      } else {
-        yn[q] = y0 + hh / T(6) * (stg[RB + n] + k);
-        const long fo = plane * P + prow0 + n;
-        if (!a.last) reinterpret_cast<T*>(a.y0)[fo] = yn[q];
-        else if (a.out_f64) reinterpret_cast<double*>(a.f_out)[fo] = double(yn[q]);
-        else reinterpret_cast<float*>(a.f_out)[fo] = yn[q];
-      }
-      if constexpr (ADJ) w[q][r] = mk<T>(px[q][r] * yn[q], py[q][r] * yn[q]);
+      for (int q = 0; q < NTI; ++q) v[q][r] = twmul<T, true>(v[q][r], w);
     }
-    if constexpr (!ADJ) w[0][r] = mk<T>(yn[0], yn[1]);
+#pragma unroll
+    for (int q = 0; q < NTI; ++q) dft<R, T, true>(v[q]);
+    // standard: v[q][r] = dx + i dy at pixel n = j + NB r of row q; adjoint: v[0][r] = (k_a, k_b)
+    if (!wait_or_record(mbar, 0)) return;  // the staged operands: recorded, drained, leave
+    const T hh = T(a.h);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      T yn[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int n = (q * LINES + line) * N + j + NB * r;  // within the block's rows
+        const T k = ADJ ? (q == 0 ? v[0][r].x : v[0][r].y) : px[q][r] * v[q][r].x + py[q][r] * v[q][r].y;
+        const T y0 = stg[n];
+        T* accg = reinterpret_cast<T*>(a.acc) + plane * P + prow0;
+        if (a.stage == 1) {
+          yn[q] = y0 + T(0.5) * hh * k;
+          accg[n] = k;
+        } else if (a.stage < 4) {
+          yn[q] = y0 + (a.stage == 2 ? T(0.5) * hh : hh) * k;
+          accg[n] = stg[RB + n] + T(2) * k;
+        } else {
+          yn[q] = y0 + hh / T(6) * (stg[RB + n] + k);
+          const long fo = plane * P + prow0 + n;
+          if (!a.last) reinterpret_cast<T*>(a.y0)[fo] = yn[q];
+          else if (a.out_f64) reinterpret_cast<double*>(a.f_out)[fo] = double(yn[q]);
+          else reinterpret_cast<float*>(a.f_out)[fo] = yn[q];
+        }
+        if constexpr (ADJ) w[q][r] = mk<T>(px[q][r] * yn[q], py[q][r] * yn[q]);
+      }
+      if constexpr (!ADJ) w[0][r] = mk<T>(yn[0], yn[1]);
+    }
+    if (a.last) return;  // uniform across the block
   }
-  if (a.last) return;  // uniform across the block
 #pragma unroll
   for (int q = 0; q < NTO; ++q) dft<R, T, false>(w[q]);  // forward pass 1 (NS = 1): outputs at 8 j + r
   __syncthreads();  // every thread has read its inverse-pass-3 inputs
