@@ -501,8 +501,11 @@ cudaError_t run_vjp_step_cluster(ClusterArgs f, ClusterArgs d, void* pp, const v
   }
   if (e != cudaSuccess) return e;
   const int g = (int)std::min<long>(((long)B * P / 2 + 255) / 256, 148L * 8);
-  return launch<k_dphi_step<T, C>>(dim3(g), 256, 0, st, (const T*)f.save, (const T*)d.save, (const T*)phi, dacc, B, P,
-                                   d.t0, d.h, flip, (int)first);
+  auto run_dphi = [&](auto minb) {
+    return launch<k_dphi_step<T, C, decltype(minb)::value>>(dim3(g), 256, 0, st, (const T*)f.save, (const T*)d.save,
+                                                            (const T*)phi, dacc, B, P, d.t0, d.h, flip, (int)first);
+  };
+  return g >= 148 * 6 ? run_dphi(std::integral_constant<int, 3>()) : run_dphi(std::integral_constant<int, 2>());
 }
 
 // The p-plane path (a.pp set) is built for float32 plans, and for float64 ones of N <= 256.

@@ -688,10 +688,13 @@ __global__ void __launch_bounds__(ClGeo<T, N, CL>::NT, MINB) k_vjp_step_cluster(
 // (lense_flow.py:195-252) with the stage weights, summed in float64.  Adjoint stage j at time t + {0, 1/2,
 // 1/2, 1} h pairs with standard stage j, or with 3 - j where that system ran the other way (``flip``).  One
 // read and one write of the five accumulators per step instead of per stage, and the 2 x 2 inverse once per
-// distinct time: bound by its bytes, 57 us a step for 16 TQU maps of 256^2 (256 MB, 4.5 TB/s) against 4 x 25 us
+// distinct time: bound by its bytes, 50 us a step for 16 TQU maps of 256^2 (256 MB, 5.1 TB/s) against 4 x 25 us
 // by stages.  grads [4][B C][2][P], inputs [4][B C][P]; two pixels per thread.
-template <typename T, int C>
-__global__ void __launch_bounds__(256) k_dphi_step(const T* __restrict__ grads, const T* __restrict__ inputs,
+// MINB 3 (80 registers, some spilled) where the grid fills the SMs several times over: reverse pass of 16 TQU maps
+// of 256^2 1,980 -> 1,930 us, 32 T maps 1,880 -> 1,778, 64 QU maps of 128^2 1,288 -> 1,252; of 4 TQU maps of 256^2
+// 569 -> 577, 2 of 128^2 206 -> 220.
+template <typename T, int C, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_dphi_step(const T* __restrict__ grads, const T* __restrict__ inputs,
                                                    const T* __restrict__ phi, double* __restrict__ acc, int B, long P,
                                                    double t, double h, int flip, int first) {
   const long planes = (long)B * C, total = (long)B * P / 2;
