@@ -456,14 +456,44 @@ template <typename T, int N> constexpr int cluster_minb() {
   return sizeof(T) == 8 ? 1 : 65536 / (ClGeo<T, N, cluster_blocks<N>()>::NT * (N == 64 ? 168 : N == 128 ? 128 : 255));
 }
 
+// A cluster writes its output plane when it is done, while other clusters may not have started: the output may
+// share memory with what they still read only plane by plane, that is in place with one type.
+inline bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+  const char *x = static_cast<const char*>(a), *y = static_cast<const char*>(b);
+  return x && y && x < y + nb && y < x + na;
+}
+// output of n pixels against an input of n pixels that every cluster reads
+inline bool clobbers(const void* out, int out64, const void* in, int in64, size_t n) {
+  return !(out == in && out64 == in64) && overlap(out, n * (out64 ? 8 : 4), in, n * (in64 ? 8 : 4));
+}
+
+// a plane buffer of T to the caller's output
+template <typename T>
+cudaError_t run_store_field(const void* src, void* dst, int dst_f64, long n, cudaStream_t st) {
+  const int g = (int)std::min<long>((n + 255) / 256, 148L * 8);
+  return launch_k<k_store_field<T>>(LF_KIND_ROW, dim3(g), 256, 0, st, static_cast<const T*>(src), dst, dst_f64, n);
+}
+
+// ``spare``: room for the fields in T; an output that other clusters' inputs share memory with goes there first.
 template <typename T, int N, bool ADJ, bool PP>
-cudaError_t run_lens_cluster(const StageArgs& a, int B, int C, int nsteps, double t0, double t1, cudaStream_t st,
-                             void* ckpt = nullptr) {
+cudaError_t run_lens_cluster(const StageArgs& a, int B, int C, int nsteps, double t0, double t1, void* spare,
+                             cudaStream_t st, void* ckpt = nullptr) {
   constexpr int CL = cluster_blocks<N>();
   ClusterArgs c = cluster_args(a, B, C, nsteps, t0, (t1 - t0) / nsteps);
   c.ckpt = ckpt;
-  return launch_clusters<k_lens_cluster<T, N, CL, ADJ, PP, cluster_minb<T, N>()>, CL>(
+  const size_t P = (size_t)N * N, n = P * B * C;
+  const void* p = PP ? a.pp : a.phi;
+  const size_t p_bytes = sizeof(T) * P * B * (PP ? 2 * (2 * (size_t)nsteps + 1) : 5);
+  const bool staged = clobbers(a.f_out, a.out_f64, a.f_in, a.in_f64, n) ||
+                      overlap(a.f_out, n * (a.out_f64 ? 8 : 4), p, p_bytes);
+  if (staged) {
+    c.f_out = spare;
+    c.out_f64 = std::is_same<T, double>::value;
+  }
+  cudaError_t e = launch_clusters<k_lens_cluster<T, N, CL, ADJ, PP, cluster_minb<T, N>()>, CL>(
       (long)B * C, ClGeo<T, N, CL>::NT, cluster_smem<T, N, CL>(), st, c);
+  if (e != cudaSuccess || !staged) return e;
+  return run_store_field<T>(spare, a.f_out, a.out_f64, (long)n, st);
 }
 
 // One step of a reverse pass on clusters: p at the step's three times (float32; into ``pp``, along ``f``),
@@ -517,9 +547,9 @@ cudaError_t run_lens_n(const StageArgs& a, int B, int nsteps, double t0, double 
         cudaError_t e = run_p_planes<T>(a, N, B, nsteps, 0.0, 1.0 / nsteps, st);
         if (e != cudaSuccess) return e;
       }
-      return run_lens_cluster<T, N, ADJ, true>(a, B, C, nsteps, t0, t1, st);
+      return run_lens_cluster<T, N, ADJ, true>(a, B, C, nsteps, t0, t1, a.y0, st);
     }
-    return run_lens_cluster<T, N, ADJ, false>(a, B, C, nsteps, t0, t1, st);
+    return run_lens_cluster<T, N, ADJ, false>(a, B, C, nsteps, t0, t1, a.y0, st);
   } else if constexpr (std::is_same<T, float>::value) {
     if (a.pp) return run_lens_pp<T, N, C, ADJ, true>(a, B, nsteps, t0, t1, st, pp_given);
     return run_lens_pp<T, N, C, ADJ, false>(a, B, nsteps, t0, t1, st);
@@ -876,9 +906,9 @@ cudaError_t run_vjp_ckpt_n(const StageArgs& af0, const StageArgs& ad0, char* ckp
       af.pp = af.y0;
       e = run_p_planes<T>(af, N, B, nsteps, 0.0, 1.0 / nsteps, st);
       if (e != cudaSuccess) return e;
-      e = run_lens_cluster<T, N, false, true>(af, B, C, nsteps, t0, t1, st, ckpt);
+      e = run_lens_cluster<T, N, false, true>(af, B, C, nsteps, t0, t1, sink, st, ckpt);
     } else {
-      e = run_lens_cluster<T, N, false, false>(af, B, C, nsteps, t0, t1, st, ckpt);
+      e = run_lens_cluster<T, N, false, false>(af, B, C, nsteps, t0, t1, sink, st, ckpt);
     }
     if (e != cudaSuccess) return e;
     ClusterArgs f = cluster_args(af0, B, C, 1, t0, h), d = cluster_args(ad0, B, C, 1, t1, hb);

@@ -670,6 +670,15 @@ __global__ void __launch_bounds__(ClGeo<T, N, CL>::NT, MINB) k_lens_cluster(Clus
   cl_integrate<T, N, CL, ADJ, PP, false>(a, blockIdx.x / CL);
 }
 
+// n pixels of T to a caller's output of either type (an output that could not be written plane by plane).
+template <typename T>
+__global__ void __launch_bounds__(256) k_store_field(const T* src, void* dst, int dst_f64, long n) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    if (dst_f64) reinterpret_cast<double*>(dst)[i] = double(src[i]);
+    else reinterpret_cast<float*>(dst)[i] = float(src[i]);
+  }
+}
+
 // Measured, reference reverse pass of 16 TQU maps of 256^2, n = 7: row, column and accumulation launches per
 // stage 3.35 ms; per step, with p formed from the derivative planes 3.1 ms, read from p planes 2.0 ms.
 //

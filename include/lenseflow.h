@@ -117,8 +117,9 @@ int lf_lense_flow_pp(lf_plan_t plan, const void* f_in, int in_dtype, void* f_out
  * (adjoint = 0) or df/dt = div(M^-1 grad(phi) f) (adjoint = 1), time running
  * 0 -> 1 iff (direction == +1) XOR adjoint.  Replaces lense_flow /
  * primal_lense_flow / single_lense_flow_step (cmb_lensing/lense_flow.py:289-352)
- * for all ``ncomp`` components of ``batch`` maps.  f_in may equal f_out.
- * ``in_dtype``/``out_dtype`` select float32/float64 field I/O. */
+ * for all ``ncomp`` components of ``batch`` maps.  f_out may share memory with
+ * f_in, in place or otherwise, also where ``in_dtype`` and ``out_dtype`` (float32
+ * or float64 field I/O) differ. */
 int lf_lense_flow(lf_plan_t plan, const void* f_in, int in_dtype, void* f_out, int out_dtype, const void* planes,
                   int batch, int nsteps, int direction, int adjoint, void* workspace, size_t workspace_bytes,
                   void* stream);
