@@ -497,18 +497,14 @@ cudaError_t run_lens_cluster(const StageArgs& a, int B, int C, int nsteps, doubl
 }
 
 // One step of a reverse pass on clusters: p at the step's three times (float32; into ``pp``, along ``f``),
-// ``f`` (standard) and ``d`` (adjoint) with their records, then the step's delta-phi terms.  The two systems run side by side unless one's output is the other's input (a
-// caller's buffers in a single-step pass): then one after the other, field first.
+// ``f`` (standard) and ``d`` (adjoint) side by side with their records, then the step's delta-phi terms.  Neither
+// system's output may share memory with what the other reads, nor its own but in place.
 template <typename T, int N, int C>
 cudaError_t run_vjp_step_cluster(ClusterArgs f, ClusterArgs d, void* pp, const void* phi, double* dacc, int B, int flip,
                                  bool first, cudaStream_t st) {
   constexpr int CL = cluster_blocks<N>();
   constexpr auto kernel = k_vjp_step_cluster<T, N, CL, cluster_minb<T, N>()>;
-  const long P = (long)N * N, n = f.planes * P;
-  auto overlap = [n](const void* a, int a64, const void* b, int b64) {
-    const char *x = static_cast<const char*>(a), *y = static_cast<const char*>(b);
-    return x && x < y + n * (b64 ? 8 : 4) && y < x + n * (a64 ? 8 : 4);
-  };
+  const long P = (long)N * N;
   cudaError_t e = cudaSuccess;
   if constexpr (std::is_same<T, float>::value) {
     StageArgs a;
@@ -521,14 +517,7 @@ cudaError_t run_vjp_step_cluster(ClusterArgs f, ClusterArgs d, void* pp, const v
     e = run_p_planes<T>(a, N, B, 1, f.t0, f.h, st);
     if (e != cudaSuccess) return e;
   }
-  const bool apart = overlap(d.f_out, d.out_f64, f.f_in, f.in_f64) || overlap(f.f_out, f.out_f64, d.f_in, d.in_f64);
-  e = launch_clusters<kernel, CL>((apart ? 1 : 2) * f.planes, ClGeo<T, N, CL>::NT, cluster_smem<T, N, CL>(),
-                                  st, f, d);
-  if (e == cudaSuccess && apart) {
-    ClusterArgs none = f;
-    none.planes = 0;
-    e = launch_clusters<kernel, CL>(d.planes, ClGeo<T, N, CL>::NT, cluster_smem<T, N, CL>(), st, none, d);
-  }
+  e = launch_clusters<kernel, CL>(2 * f.planes, ClGeo<T, N, CL>::NT, cluster_smem<T, N, CL>(), st, f, d);
   if (e != cudaSuccess) return e;
   const int g = (int)std::min<long>(((long)B * P / 2 + 255) / 256, 148L * 8);
   auto run_dphi = [&](auto minb) {
@@ -770,6 +759,17 @@ cudaError_t run_vjp_n(const StageArgs& af0, const StageArgs& ad0, double* dacc, 
     f.save = af0.y0;
     d.save = static_cast<char*>(af0.y0) + 8 * plane;
     void* pp = static_cast<char*>(ad0.between) + plane;
+    // A caller's output that shares memory with what the last step still reads leaves it through the buffers
+    // between the steps: the other system's input (or, not in place, its own) in a single step, the
+    // derivative planes always.
+    const size_t n = (size_t)B * C * P;
+    auto staged = [&](const StageArgs& o) {
+      return (nsteps == 1 && (clobbers(o.f_out, o.out_f64, o.f_in, o.in_f64, n) ||
+                              overlap(o.f_out, n * (o.out_f64 ? 8 : 4), (&o == &af0 ? ad0 : af0).f_in,
+                                      n * (o.in_f64 ? 8 : 4)))) ||
+             overlap(o.f_out, n * (o.out_f64 ? 8 : 4), af0.phi, sizeof(T) * 5 * (size_t)B * P);
+    };
+    const bool want_f = af0.f_out != af0.between, stage_f = want_f && staged(af0), stage_d = staged(ad0);
     for (int i = 0; i < nsteps; ++i) {
       const bool last = i == nsteps - 1;
       f.t0 = d.t0 = t0 + i * h;
@@ -778,14 +778,19 @@ cudaError_t run_vjp_n(const StageArgs& af0, const StageArgs& ad0, double* dacc, 
         d.f_in = ad0.between;
         f.in_f64 = d.in_f64 = io64;
       }
-      f.f_out = !last ? af0.between : af0.f_out == af0.between ? nullptr : af0.f_out;
-      d.f_out = !last ? ad0.between : ad0.f_out;
-      f.out_f64 = last ? af0.out_f64 : io64;
-      d.out_f64 = last ? ad0.out_f64 : io64;
+      const bool to_f = last && !stage_f, to_d = last && !stage_d;
+      f.f_out = !to_f ? af0.between : want_f ? af0.f_out : nullptr;
+      d.f_out = !to_d ? ad0.between : ad0.f_out;
+      f.out_f64 = to_f ? af0.out_f64 : io64;
+      d.out_f64 = to_d ? ad0.out_f64 : io64;
       cudaError_t e = run_vjp_step_cluster<T, N, C>(f, d, pp, af0.phi, dacc, B, 0, i == 0, st);
       if (e != cudaSuccess) return e;
     }
-    return cudaSuccess;
+    if (stage_f) {
+      cudaError_t e = run_store_field<T>(af0.between, af0.f_out, af0.out_f64, (long)n, st);
+      if (e != cudaSuccess) return e;
+    }
+    return stage_d ? run_store_field<T>(ad0.between, ad0.f_out, ad0.out_f64, (long)n, st) : cudaSuccess;
   } else {
   const double hh = h / 2.0;
   const double cw[4] = {1.0, 2.0, 2.0, 1.0};
@@ -916,9 +921,12 @@ cudaError_t run_vjp_ckpt_n(const StageArgs& af0, const StageArgs& ad0, char* ckp
     f.f_out = nullptr;
     f.save = grads;
     d.save = ad0.y0;
+    const size_t nf = (size_t)B * C * P;
+    const bool stage_d = (nsteps == 1 && clobbers(ad0.f_out, ad0.out_f64, ad0.f_in, ad0.in_f64, nf)) ||
+                         overlap(ad0.f_out, nf * (ad0.out_f64 ? 8 : 4), af0.phi, sizeof(T) * 5 * (size_t)B * P);
     for (int ib = 0; ib < nsteps; ++ib) {
       const int i = nsteps - 1 - ib;
-      const bool last = ib == nsteps - 1;
+      const bool to_d = ib == nsteps - 1 && !stage_d;
       f.f_in = ckpt + (size_t)i * plane;
       f.t0 = t0 + i * h;
       d.t0 = t0 + (i + 1) * h;
@@ -926,12 +934,12 @@ cudaError_t run_vjp_ckpt_n(const StageArgs& af0, const StageArgs& ad0, char* ckp
         d.f_in = ad0.between;
         d.in_f64 = io64;
       }
-      d.f_out = last ? ad0.f_out : ad0.between;
-      d.out_f64 = last ? ad0.out_f64 : io64;
+      d.f_out = to_d ? ad0.f_out : ad0.between;
+      d.out_f64 = to_d ? ad0.out_f64 : io64;
       e = run_vjp_step_cluster<T, N, C>(f, d, af0.between, af0.phi, dacc, B, 1, ib == 0, st);
       if (e != cudaSuccess) return e;
     }
-    return cudaSuccess;
+    return stage_d ? run_store_field<T>(ad0.between, ad0.f_out, ad0.out_f64, (long)nf, st) : cudaSuccess;
   } else {
   // ---- forward integration, storing y_i at the start of each step
   af.h = h;

@@ -145,7 +145,8 @@ int lf_irfft2(lf_plan_t plan, const void* spec, int batch, void* maps, int out_d
  * (before undo_inner_product), optional ``f_back`` (the re-integrated field),
  * and ``dphi``: [batch][N][N/2+1] complex128 if dphi_basis = LF_PHI_FOURIER
  * (accumulated in Fourier space, lense_flow.py:233-239) or [batch][N][N]
- * float64 if LF_PHI_MAP (lense_flow.py:240-248). */
+ * float64 if LF_PHI_MAP (lense_flow.py:240-248).  ``delta_f`` may share memory
+ * with any input, ``f_back`` with ``f_lensed`` and ``cotangent``. */
 size_t lf_vjp_workspace_bytes(lf_plan_t plan, int batch);
 int lf_lense_flow_vjp(lf_plan_t plan, const void* f_lensed, const void* cotangent, int io_dtype, const void* planes,
                       int batch, int nsteps, int direction, void* delta_f, void* f_back, void* dphi, int dphi_basis,

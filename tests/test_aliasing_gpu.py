@@ -95,3 +95,59 @@ def test_noalloc_in_place_between_types(torch_cuda):
                                                   ptr(planes), B, n, 1, 0, st))
     torch.cuda.synchronize()
     assert torch.equal(out, want)
+
+
+def _reverse(torch, scheme, plan, B, n, f, cot, planes, out, other, dphi, io):
+    """lf_lense_flow_vjp (``other``: the re-integrated field) or lf_lense_flow_vjp_ckpt (``other``: the lensed field)."""
+    from cmblensing_b200 import _native as nat
+    lib, ptr = plan._lib, lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    if scheme == "exact":
+        nbytes = lib.lf_vjp_ckpt_workspace_bytes(plan.handle, B, n)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+        nat.check(lib.lf_lense_flow_vjp_ckpt(plan.handle, ptr(f), ptr(cot), io, ptr(planes), B, n, 1, ptr(other), ptr(out),
+                                             ptr(dphi), nat.LF_PHI_FOURIER, ptr(ws), nbytes, st))
+    else:
+        nbytes = lib.lf_vjp_workspace_bytes(plan.handle, B)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+        nat.check(lib.lf_lense_flow_vjp(plan.handle, ptr(f), ptr(cot), io, ptr(planes), B, n, 1, ptr(out), ptr(other),
+                                        ptr(dphi), nat.LF_PHI_FOURIER, ptr(ws), nbytes, st))
+    torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("N,B", [(64, 90), (256, 7)])
+@pytest.mark.parametrize("io64", [False, True])
+@pytest.mark.parametrize("case", ["back over cotangent", "swapped", "delta one map on", "delta over planes",
+                                  "exact: delta one map on", "exact: delta over planes"])
+@pytest.mark.parametrize("n", [1, 2])
+def test_reverse_pass_outputs_over_inputs(torch_cuda, N, B, io64, case, n):
+    """The two systems of a reverse step run side by side: outputs over the other system's input (a single step reads
+    it until its end), over a neighbour's plane, over the derivative planes (read until the last delta-phi terms)."""
+    torch = torch_cuda
+    from cmblensing_b200 import _native as nat
+    C = 2
+    scheme = "exact" if case.startswith("exact") else "reference"
+    plan, f, phi = _problem(torch, N, B, C)
+    dt, io = (torch.float64, nat.LF_F64) if io64 else (torch.float32, nat.LF_F32)
+    f = f.to(dt)
+    cot = f.flip(0).flip(-1).contiguous()
+    planes = plan.phi_planes(phi)
+    dphi = torch.empty((B, N, N // 2 + 1), dtype=torch.complex128, device="cuda")
+    want, other, want_dphi = torch.empty_like(f), torch.empty_like(f), torch.empty_like(dphi)
+    _reverse(torch, scheme, plan, B, n, f, cot, planes, want, other, want_dphi, io)
+    fi, ci, pi = f.clone(), cot.clone(), planes.clone()
+    out, back = torch.empty_like(f), None
+    if case == "back over cotangent":
+        back = ci
+    elif case == "swapped":
+        out, back = fi, ci
+    elif case.endswith("one map on"):
+        buf = torch.empty((B + 1, C, N, N), dtype=dt, device="cuda")
+        buf[:B] = cot
+        ci, out = buf[:B], buf[1:]
+    else:
+        out = pi.view(-1).view(dt)[:f.numel()].view(f.shape)
+    _reverse(torch, scheme, plan, B, n, fi, ci, pi, out, back, dphi, io)
+    assert torch.equal(out, want) and torch.equal(dphi, want_dphi)
+    if back is not None:
+        assert torch.equal(back, other)
