@@ -331,9 +331,9 @@ cudaError_t run_lens_pp(const StageArgs& base, int B, int nsteps, double t0, dou
   a.pp_idx = pidx(0);
   // Programmatic dependent launch for small batches (up to 2^23 pixels, 16 maps of 512^2 QU):
   // measured per 512^2 QU lens with the phi precompute, 4 maps 0.79 -> 0.66 ms, 16 maps 2.35 ->
-  // 2.25 ms, but 64 maps 7.85 -> 8.13 ms.  The initial transform follows k_p_planes (which has no
-  // dependency wait) or the caller's work and is launched plainly; every later stage kernel waits
-  // for its predecessor itself.
+  // 2.25 ms, but 64 maps 7.85 -> 8.13 ms.  Every stage kernel waits for its predecessor itself, the initial
+  // transform on the p-plane path among them (its predecessor, k_p_planes or the caller's work, triggers
+  // nothing early); the initial transform that reads no p planes is launched plainly.
   const bool use_pdl = (long)B * C * N * N <= (1L << 23);
   PdlScope pdl;
   if (PP && use_pdl) pdl.enable();

@@ -535,7 +535,6 @@ __device__ __forceinline__ void cl_integrate(const ClusterArgs& a, long cmap) {
     sys.init_barriers();
   }
   const int polls = g_lf_wait_polls;
-  pdl_wait();
   const int lane = sys.lane;
   const long r0 = (long)rank * G::RPC + 2 * sys.g;  // first row of this group's pair
   const T ky_scale = T(a.kbase / double(N));

@@ -122,8 +122,15 @@ __device__ __forceinline__ void load_twiddles(c2<T>* tw, const void* g, int tid)
 // Programmatic dependent launch.  A stage kernel lets the next kernel of the
 // stream launch once all its blocks are running (its blocks then fill SMs as
 // this grid drains), and waits for the previous kernel to complete, with its
-// memory visible, before touching any buffer the two share.  Without the
-// launch attribute both are no-ops.
+// memory visible, before touching any buffer the two share.  What it reads
+// after the wait it reads with ordinary loads: a non-coherent one (__ldg, a
+// __restrict__ const parameter) is only defined for memory that stays constant
+// for the kernel's whole life, and the compiler may move it ahead of the wait.
+// The p planes qualify in the stage kernels k_row_pair and k_row_pair_adj:
+// their writer triggers nothing early, so it is done before the lens's first
+// kernel starts, and the stage kernels start after that one (the adjoint lens
+// of 8 QU maps of 512^2 983 us, with ordinary loads there 1,015).
+// Without the launch attribute both are no-ops.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -959,8 +966,8 @@ __global__ void __launch_bounds__(NT, MINB) k_row_rows(StageArgs a) {
     for (int q = 0; q < 2; ++q)
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        px[q][r] = __ldg(pq + q * LINES * N + NB * r);
-        py[q][r] = __ldg(pq + P + q * LINES * N + NB * r);
+        px[q][r] = pq[q * LINES * N + NB * r];
+        py[q][r] = pq[P + q * LINES * N + NB * r];
       }
   }
   const c2<T>* tw2 = tw;                      // (RM, 8)
