@@ -170,6 +170,15 @@ template <int CL> __device__ __forceinline__ void cluster_sync() {
   }
 }
 
+// The way out of a warp whose wait ran out.  The cluster's other warps miss its puts, so that their own next wait
+// runs out too: each waits once more at most (about two seconds with its drain), puts nothing after that and comes
+// here or has finished.  The barrier, which threads that have exited do not hold up, keeps every block's shared
+// memory until the last put into it has been sent and drained.
+__device__ __forceinline__ void cluster_leave() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // ------------------------------------------------------ group transforms
 // One radix-R pass on registers: butterfly i of a lane is b = lane + TP i, its input r in register i + (E/R) r.
 template <typename T, int N, int R, int NS, bool INV, int E>
@@ -302,17 +311,22 @@ template <typename T, int N, int CL> struct ClSystem {
       }
     }
   }
-  // All of area ``which`` has landed for phase number ``phase``; ``more``: another phase follows.
-  __device__ __forceinline__ void landed(int which, int phase, int polls, bool more) const {
+  // All of area ``which`` has landed for phase number ``phase``; ``more``: another phase follows.  False, for the
+  // whole warp, if a lane's wait ran out: recorded, then drained like wait_or_record, and the warp leaves by
+  // cluster_leave.
+  __device__ __forceinline__ bool landed(int which, int phase, int polls, bool more) const {
     if constexpr (CL > 1) {
-      if (!cluster_mbar_wait(mbar + which, phase & 1, polls)) {  // recorded; then drained like wait_or_record
+      const bool ok = cluster_mbar_wait(mbar + which, phase & 1, polls);
+      if (!ok) {
         record_timeout();
         cluster_mbar_wait(mbar + which, phase & 1, kWaitTries);
       }
+      if (!__all_sync(0xffffffffu, ok)) return false;
       if (threadIdx.x == 0 && more) mbar_expect_tx(mbar + which, kPhaseBytes);
     } else {
       __syncthreads();
     }
+    return true;
   }
   __device__ __forceinline__ void put(c2<T>* local, uint32_t to, int which, c2<T> v) const {
     if constexpr (CL == 1) *local = v;
@@ -588,7 +602,7 @@ __device__ __forceinline__ void cl_integrate(const ClusterArgs& a, long cmap) {
   int k_now = -1;
   if constexpr (SAVE && ADJ) store(save, y0);
   cluster_sync<CL>();       // every block runs, with its barriers initialised, before anyone puts into it
-  wait_or_record(mbar, 0);  // (a timed-out wait is recorded; the block goes on, as at every wait below)
+  wait_or_record(mbar, 0);  // (a timed-out wait is recorded; the block goes on to its next wait)
   if constexpr (ADJ) {
     load_p(0);
     k_now = 0;
@@ -607,7 +621,7 @@ __device__ __forceinline__ void cl_integrate(const ClusterArgs& a, long cmap) {
     if constexpr (!ADJ && !SAVE) {
       if (s == 0 && a.ckpt) store(reinterpret_cast<T*>(a.ckpt) + ((it >> 2) * a.planes + cmap) * P, y0);
     }
-    sys.landed(0, it, polls, !last);
+    if (!sys.landed(0, it, polls, !last)) return cluster_leave();
     // p at the rate's time (standard) or at the next stage's (adjoint), needed when the columns have landed
     const int k = ADJ ? i2 + (s < 2 ? 1 : 2) : i2 + (s == 0 ? 0 : s < 3 ? 1 : 2);
     sys.columns(kxs, [&]() {
@@ -616,7 +630,7 @@ __device__ __forceinline__ void cl_integrate(const ClusterArgs& a, long cmap) {
         k_now = k;
       }
     });
-    sys.landed(1, it, polls, !last);
+    if (!sys.landed(1, it, polls, !last)) return cluster_leave();
     T yn[2][E];
     if constexpr (ADJ) {
       c2<T> v[1][E];
@@ -651,7 +665,7 @@ __device__ __forceinline__ void cl_integrate(const ClusterArgs& a, long cmap) {
       sys.forward_std(yn[0], yn[1]);
     }
   }
-  // (nothing is put into a block after its last Gx area has landed, so it may exit)
+  // (nothing is put into a block after its last Gx area has landed whole, so it may exit)
   if (!a.f_out) return;
 #pragma unroll
   for (int q = 0; q < 2; ++q)

@@ -209,10 +209,12 @@ int lf_lense_flow_noalloc(int nside, int ncomp, double pix_width, const void* f_
                           void* stream);
 
 /* Device-wait timeouts.  Every wait of a kernel block on its own bulk copies
- * into shared memory is bounded (about one second of polls).  A block whose
- * wait runs out records it, waits once more (bounded) for its copies in
- * flight and then skips or finishes its work: the results of that launch and
- * of everything computed from them are invalid.  The record is sticky: from
+ * into shared memory, or on what the other blocks of its cluster store there
+ * (N <= 256), is bounded (about one second of polls).  A block whose wait runs
+ * out records it, waits once more (bounded) for its copies in flight and then
+ * skips or finishes its work; on a cluster it stops, writes no output, and the
+ * cluster's other blocks stop at their next wait (a few seconds in all).  The
+ * results of that launch and of everything computed from them are invalid.  The record is sticky: from
  * then on every computing entry point (lf_phi_precompute, lf_lense_flow,
  * lf_lense_flow_vjp, lf_rfft2, lf_irfft2, lf_lense_flow_noalloc) returns
  * LF_ERR_TIMEOUT without launching anything, until lf_wait_timeouts resets
