@@ -1133,14 +1133,6 @@ __global__ void __launch_bounds__(NT, MINB) k_row_rows(StageArgs a) {
 // :398-415), at the K = 2n+1 stage times t_k = t0 + k hh of an RK4
 // integration, from the five derivative planes; float64 arithmetic, stored in
 // T.  grid: x covers P/2 pixel pairs, y = map.
-// Float32 planes go through the adjugate of the symmetric 2 x 2 M, as in
-// k_phi_rows_c2r_pp: with b_x = H_yy phi_x - H_xy phi_y, b_y = H_xx phi_y -
-// H_xy phi_x, l = tr H and q = det H formed once per pixel,
-// p = (grad phi + t b) / (1 + t l + t^2 q + 1e-12), the reciprocal as its float32
-// approximation and one float64 Newton step (2^-44).  The float64 pipe bound
-// the direct form (inverse matrix and a full division at every time).
-// Float64 planes keep it: their values are those that the kernels form from
-// the derivative planes, bit for bit.
 template <typename T>
 __global__ void __launch_bounds__(256) k_p_planes(const T* __restrict__ planes, T* __restrict__ pp, long P, int K,
                                                   double t0, double hh) {
@@ -1151,35 +1143,11 @@ __global__ void __launch_bounds__(256) k_p_planes(const T* __restrict__ planes, 
     c2<T> f[5];
 #pragma unroll
     for (int j = 0; j < 5; ++j) f[j] = reinterpret_cast<const c2<T>*>(ph + j * P)[i];
-    double gx[2], gy[2], bx[2], by[2], l[2], q[2];
-    if constexpr (sizeof(T) == 4) {
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        gx[u] = u ? f[0].y : f[0].x;
-        gy[u] = u ? f[1].y : f[1].x;
-        const double A = u ? f[2].y : f[2].x, B = u ? f[3].y : f[3].x, Cc = u ? f[4].y : f[4].x;
-        bx[u] = Cc * gx[u] - B * gy[u];
-        by[u] = A * gy[u] - B * gx[u];
-        l[u] = A + Cc;
-        q[u] = A * Cc - B * B;
-      }
-    }
     for (int k = 0; k < K; ++k) {
       const double t = t0 + k * hh;
       double ox[2], oy[2];
-      if constexpr (sizeof(T) == 4) {
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const double D = fma(t, fma(t, q[u], l[u]), 1.0 + 1e-12);
-          double r = double(rcp_approx(float(D)));
-          r = fma(r, fma(-D, r, 1.0), r);
-          ox[u] = fma(t, bx[u], gx[u]) * r;
-          oy[u] = fma(t, by[u], gy[u]) * r;
-        }
-      } else {
-        p_vector<double>(f[0].x, f[1].x, f[2].x, f[3].x, f[4].x, t, ox[0], oy[0]);
-        p_vector<double>(f[0].y, f[1].y, f[2].y, f[3].y, f[4].y, t, ox[1], oy[1]);
-      }
+      p_vector<double>(f[0].x, f[1].x, f[2].x, f[3].x, f[4].x, t, ox[0], oy[0]);
+      p_vector<double>(f[0].y, f[1].y, f[2].y, f[3].y, f[4].y, t, ox[1], oy[1]);
       reinterpret_cast<c2<T>*>(out + (2 * k) * P)[i] = mk<T>(T(ox[0]), T(ox[1]));
       reinterpret_cast<c2<T>*>(out + (2 * k + 1) * P)[i] = mk<T>(T(oy[0]), T(oy[1]));
     }
