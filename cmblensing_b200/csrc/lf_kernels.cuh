@@ -1475,10 +1475,9 @@ __global__ void __launch_bounds__(NT, N == 1024 ? 2 : 4) k_phi_rows_c2r_pp(const
     //   p_x = (phi_x + t (H_yy phi_x - H_xy phi_y)) / D,  p_y = (phi_y + t (H_xx phi_y - H_xy phi_x)) / D,
     //   D = det M = 1 + t (H_xx + H_yy) + t^2 (H_xx H_yy - H_xy^2).
     // The time-independent coefficients are formed once per pixel in float64; each time then costs two
-    // FMAs for D, a reciprocal and four FMA/multiplies in float32 (the RK4 right-hand side that reads the
-    // planes is float32), on pixel pairs in packed arithmetic.  The reference's det + 1e-12
-    // (lense_flow.py:408-411) is below float32 resolution for D >= 0.2 and is not added.  (Scalar, with
-    // correctly rounded reciprocals, the loop was a third of this pass's 684 instructions per pixel.)
+    // FMAs for D, a correctly rounded reciprocal and four FMA/multiplies in float32 (the RK4 right-hand side
+    // that reads the planes is float32), on pixel pairs in packed arithmetic (the same bits as scalar).  The
+    // reference's det + 1e-12 (lense_flow.py:408-411) is below float32 resolution for D >= 0.2 and is not added.
     float2 gx[2], gy[2], bx[2], by[2], lt[2], qt[2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
@@ -1498,15 +1497,24 @@ __global__ void __launch_bounds__(NT, N == 1024 ? 2 : 4) k_phi_rows_c2r_pp(const
     for (int k = 0; k < K; ++k) {
       const float t = float(double(k) * inv2n);
       const float2 tt = make_float2(t, t);
-      float2 ox[2], oy[2];
+      float2 D[2], r[2], ox[2], oy[2];
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        const float2 D = f2_fma(tt, f2_fma(tt, qt[q], lt[q]), one);
-        // 1 / D: the hardware approximation and one Newton step, r + r (1 - D r)
-        float2 r = make_float2(rcp_approx(D.x), rcp_approx(D.y));
-        r = f2_fma(r, f2_fma(make_float2(-D.x, -D.y), r, one), r);
-        ox[q] = f2_mul(f2_fma(tt, bx[q], gx[q]), r);
-        oy[q] = f2_mul(f2_fma(tt, by[q], gy[q]), r);
+        D[q] = f2_fma(tt, f2_fma(tt, qt[q], lt[q]), one);
+        // 1 / D, correctly rounded: the hardware approximation and one Newton step, r + r (1 - D r), give __frcp_rn's
+        // bits for every mantissa and all |D| from 2^-47 (D = 1 + ... is no smaller) to 2^126
+        r[q] = make_float2(rcp_approx(D[q].x), rcp_approx(D[q].y));
+        r[q] = f2_fma(r[q], f2_fma(make_float2(-D[q].x, -D[q].y), r[q], one), r[q]);
+      }
+      const float2 rr = f2_mul(r[0], r[1]);
+      if (!(fabsf(rr.x * rr.y) > 0.0f)) {  // zero or NaN: D is zero, huge, infinite or NaN somewhere
+#pragma unroll
+        for (int q = 0; q < 2; ++q) r[q] = make_float2(__frcp_rn(D[q].x), __frcp_rn(D[q].y));
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        ox[q] = f2_mul(f2_fma(tt, bx[q], gx[q]), r[q]);
+        oy[q] = f2_mul(f2_fma(tt, by[q], gy[q]), r[q]);
       }
       *reinterpret_cast<float4*>(out + (2 * k) * P) = make_float4(ox[0].x, ox[0].y, ox[1].x, ox[1].y);
       *reinterpret_cast<float4*>(out + (2 * k + 1) * P) = make_float4(oy[0].x, oy[0].y, oy[1].x, oy[1].y);
