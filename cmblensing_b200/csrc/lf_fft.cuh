@@ -162,24 +162,34 @@ template <typename T, bool INV> LF_HD void dft8(c2<T>* a) {
   a[7] = caxpy<T>(-c, s3, e[3]);
 }
 
-// a <- a + w b, b <- a - w b for a constant twiddle w = (wr, wi), with FMAs: w b is written as
-// wr (1 + i wi/wr) b when |wr| >= |wi|, else wi (wr/wi + i) b, so the scaled b costs two FMAs and
-// each output two more (six instructions instead of eight for a multiply, then an add and a subtract).
+// A constant twiddle w = wr + i wi as f (1 + i t), f = wr (``re``), or as f (t + i), f = wi: an equal number of
+// operations, but the rounded f and f t are off by different amounts.  A constant's error is the same in every
+// transform and adds up over the stages of a lens, unlike the roundings of the data, so the form whose constants
+// come out closer is taken, with t the quotient by the rounded f.  Units of 2^-24, nearest f and wi / wr of the
+// larger part -> this: pi/16 0.51 -> 0.04, pi/8 0.49 -> 0.37, 3 pi/16 0.55 -> 0.29.  Relative error of float32
+// lenses, n = 7, against the float64 engine: T 256^2 9.2e-8 -> 8.5e-8, QU 512^2 9.7e-8 -> 9.3e-8, TQU 1024^2
+// 1.09e-7 -> 1.00e-7, adjoint TQU 1024^2 1.25e-7 -> 1.17e-7.
+template <typename T> struct TwForm {
+  T f, t;
+  bool re;
+};
+template <typename T> __host__ __device__ constexpr double tw_error(double f, double g) {  // squared, of f and g = f t
+  const double a = double(T(f)), b = a * double(T(g / a));
+  return (a - f) * (a - f) + (b - g) * (b - g);
+}
+template <typename T> __host__ __device__ constexpr TwForm<T> tw_form(double wr, double wi) {
+  if (tw_error<T>(wr, wi) <= tw_error<T>(wi, wr)) return TwForm<T>{T(wr), T(wi / double(T(wr))), true};
+  return TwForm<T>{T(wi), T(wr / double(T(wi))), false};
+}
+
+// a <- a + w b, b <- a - w b for a constant twiddle w = (wr, wi), with FMAs: the scaled b costs two and each
+// output two more (six instructions instead of eight for a multiply, then an add and a subtract).
 template <typename T> LF_HD void bfly_w(c2<T>& a, c2<T>& b, double wr, double wi) {
-  c2<T> u;
-  T f;
-  if (wr * wr >= wi * wi) {
-    const T t = T(wi / wr);
-    u = mk<T>(b.x - t * b.y, b.y + t * b.x);
-    f = T(wr);
-  } else {
-    const T t = T(wr / wi);
-    u = mk<T>(t * b.x - b.y, t * b.y + b.x);
-    f = T(wi);
-  }
+  const TwForm<T> w = tw_form<T>(wr, wi);
+  const c2<T> u = w.re ? mk<T>(b.x - w.t * b.y, b.y + w.t * b.x) : mk<T>(w.t * b.x - b.y, w.t * b.y + b.x);
   const c2<T> a0 = a;
-  a = caxpy<T>(f, u, a0);
-  b = caxpy<T>(-f, u, a0);
+  a = caxpy<T>(w.f, u, a0);
+  b = caxpy<T>(-w.f, u, a0);
 }
 
 // Radix-2 split into two 8-point DFTs: X[k] = E[k] + W16^k O[k], X[k+8] = E[k] - W16^k O[k].
