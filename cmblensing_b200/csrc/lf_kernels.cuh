@@ -126,10 +126,11 @@ __device__ __forceinline__ void load_twiddles(c2<T>* tw, const void* g, int tid)
 // after the wait it reads with ordinary loads: a non-coherent one (__ldg, a
 // __restrict__ const parameter) is only defined for memory that stays constant
 // for the kernel's whole life, and the compiler may move it ahead of the wait.
-// The p planes qualify in the stage kernels k_row_pair and k_row_pair_adj:
-// their writer triggers nothing early, so it is done before the lens's first
-// kernel starts, and the stage kernels start after that one (the adjoint lens
-// of 8 QU maps of 512^2 983 us, with ordinary loads there 1,015).
+// The p planes qualify in the stage kernels (k_row_pair, k_row_pair_adj and
+// k_row_rows, but for its INIT form): their writer triggers nothing early, so
+// it is done before the lens's first kernel starts, and the stage kernels start
+// after that one.  With ordinary loads there the adjoint lens of 8 QU maps of
+// 512^2 takes 1,015 us instead of 983, the lens of 16 T maps 1,005 instead of 963.
 // Without the launch attribute both are no-ops.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -966,8 +967,8 @@ __global__ void __launch_bounds__(NT, MINB) k_row_rows(StageArgs a) {
     for (int q = 0; q < 2; ++q)
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        px[q][r] = pq[q * LINES * N + NB * r];
-        py[q][r] = pq[P + q * LINES * N + NB * r];
+        px[q][r] = INIT ? pq[q * LINES * N + NB * r] : __ldg(pq + q * LINES * N + NB * r);
+        py[q][r] = INIT ? pq[P + q * LINES * N + NB * r] : __ldg(pq + P + q * LINES * N + NB * r);
       }
   }
   const c2<T>* tw2 = tw;                      // (RM, 8)

@@ -23,8 +23,8 @@ def _kernels():
 
 def test_no_noncoherent_loads_behind_the_wait():
     """A non-coherent load needs memory that is constant for the kernel's whole life and may move ahead of
-    griddepcontrol.wait: neither __ldg nor a __restrict__ parameter in a kernel that waits.  The p planes in the two
-    paired stage kernels are constant from before the lens's first kernel started."""
+    griddepcontrol.wait: neither __ldg nor a __restrict__ parameter in a kernel that waits.  The p planes are constant
+    from before the lens's first kernel started, and so in the stage kernels that follow it."""
     kernels = _kernels()
     waiting = {k: v for k, v in kernels.items() if "pdl_wait()" in v[1]}
     assert {"k_col", "k_row", "k_row_pair", "k_row_pair_adj", "k_row_rows"} <= set(waiting)
@@ -32,4 +32,6 @@ def test_no_noncoherent_loads_behind_the_wait():
         assert "__restrict__" not in params and "ld.global.nc" not in body, name
         if name in ("k_row_pair", "k_row_pair_adj"):
             body = body.replace("__ldg(pq + ", "")
+        if name == "k_row_rows":
+            body = re.sub(r"INIT \? pq\[([^]]*)\] : __ldg\(pq \+ \1\)", "", body)
         assert "__ldg" not in body, name
