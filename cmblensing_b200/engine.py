@@ -368,10 +368,11 @@ class HostPipeline:
     Each call copies f [B,C,N,N] and phi [B,N,N] (pinned host memory) to the
     device, computes the phi derivative planes (with the magnification check),
     lenses, and copies the result back into a pinned host buffer.  The batch
-    is split into ``chunks`` (the default takes fewer for small calls, see
-    ``default_chunks``; any other number is taken as given) that move through ``slots`` sets of device
-    buffers: host-to-device copies on one stream, compute alternating between
-    ``compute_streams`` streams, device-to-host copies on another.  A chunk's
+    is split into ``chunks`` (a number is taken as given; None asks
+    ``default_chunks``, which takes fewer for small calls) that move through
+    ``slots`` sets of device buffers: host-to-device copies on one stream,
+    compute alternating between ``compute_streams`` streams, device-to-host
+    copies on another.  A chunk's
     lens is a few dozen short launches; with two compute streams the kernels
     of neighbouring chunks fill each other's tail waves and launch gaps, so
     smaller chunks (better copy overlap) stop costing compute throughput.
@@ -399,14 +400,14 @@ class HostPipeline:
     is known).
     """
 
-    def __init__(self, plan, batch, io_dtype=torch.float64, chunks=DEFAULT_CHUNKS, compute_streams=2, slots=4,
+    def __init__(self, plan, batch, io_dtype=torch.float64, chunks=None, compute_streams=2, slots=4,
                  use_graphs=True, chunk_sizes=None):
         self.plan = plan
         N, C = plan.nside, plan.ncomp
         dev = plan.device
         self.batch = batch
         self.io_dtype = io_dtype
-        if chunk_sizes is None and chunks == DEFAULT_CHUNKS:
+        if chunks is None:
             chunks = default_chunks(self.h2d_bytes())
         chunk_sizes = chunk_schedule(batch, chunks, chunk_sizes)
         self.sizes = chunk_sizes
