@@ -204,8 +204,12 @@ class Plan:
         # a caller's workspace of at least the minimum is used as given (the
         # engine reads the p planes only when it also has room for them)
         if workspace is None or workspace.numel() < self.workspace_bytes(B, adjoint):
-            workspace = torch.empty(max(self.workspace_bytes(B, adjoint, n), 16), dtype=torch.uint8,
-                                    device=self.device)
+            try:
+                workspace = torch.empty(max(self.workspace_bytes(B, adjoint, n), 16), dtype=torch.uint8,
+                                        device=self.device)
+            except torch.OutOfMemoryError:  # no room for the p planes: form p in every stage
+                workspace = torch.empty(max(self.workspace_bytes(B, adjoint), 16), dtype=torch.uint8,
+                                        device=self.device)
         code = lambda t: nat.LF_F64 if t == torch.float64 else nat.LF_F32
         with torch.cuda.device(self.device):
             nat.check(self._lib.lf_lense_flow(self.handle, _ptr(f), code(f.dtype), _ptr(out), code(out.dtype),
