@@ -299,7 +299,7 @@ cudaError_t run_p_planes(const StageArgs& a, int N, int B, int nsteps, double t0
 
 // The p planes hold p = M(t)^-1 grad(phi) at the 2n+1 times k / (2n), k = 0..2n, ascending; an
 // integration from t0 = 1 reads time t0 + k hh at index 2n - k.  ``pp_given``: the caller supplies
-// them (lf_lense_flow_pp), otherwise k_p_planes forms them from the derivative planes first.
+// them (lf_lense_flow_pp), otherwise k_p_planes forms them from the derivative planes first.  PP: float32 only.
 template <typename T, int N, int C, bool ADJ, bool PP>
 cudaError_t run_lens_pp(const StageArgs& base, int B, int nsteps, double t0, double t1, cudaStream_t st,
                         bool pp_given = false) {
@@ -337,12 +337,12 @@ cudaError_t run_lens_pp(const StageArgs& base, int B, int nsteps, double t0, dou
   const bool use_pdl = (long)B * C * N * N <= (1L << 23);
   PdlScope pdl;
   if (PP && use_pdl) pdl.enable();
-  if constexpr (PP && std::is_same<T, float>::value) {
+  if constexpr (PP && N >= 512) {
     constexpr int PL = 1024 / N, PNT = (N / 8) * PL;
     e = launch_k<k_row_rows<N, PL, PNT, 6, ADJ, true>>(LF_KIND_ROW, dim3(N / (2 * PL), B * C), PNT,
                                                        row_rows_smem_bytes<N, PL>(true), st, a);
   } else {
-    e = launch_k<k_row<T, N, C, ADJ, true, RL, RNT, false, RMB>>(LF_KIND_ROW, grow, RNT, smem_row, st, a);
+    e = launch_k<k_row<T, N, C, ADJ, true, RL, RNT, false, RMB, PP>>(LF_KIND_ROW, grow, RNT, smem_row, st, a);
   }
   if (e != cudaSuccess) return e;
   if (use_pdl) pdl.enable();
@@ -361,26 +361,26 @@ cudaError_t run_lens_pp(const StageArgs& base, int B, int nsteps, double t0, dou
       a.last = (i == nsteps - 1 && s == 3);
       e = launch_col<T, N>(B * C, st, a);
       if (e != cudaSuccess) return e;
-      if constexpr (PP && C == 2 && !ADJ && N == 512 && std::is_same<T, float>::value) {
+      if constexpr (PP && C == 2 && !ADJ && N == 512) {
         // two components: full-length complex transforms, update fused in registers;
         // 2-row tiles, 128 threads (measured best of 1, 2 and 4 rows: 6.81, 5.48 and
         // 5.96 ms of row passes per 64-map step), six blocks per SM
         constexpr int PL = 2, PNT = (N / 8) * PL;
         e = launch_k<k_row_pair<N, PL, PNT, 6>>(LF_KIND_ROW, dim3(N / PL, B), PNT, row_pair_smem_bytes<PL>(N),
                                                 st, a);
-      } else if constexpr (PP && C == 2 && ADJ && N == 512 && std::is_same<T, float>::value) {
+      } else if constexpr (PP && C == 2 && ADJ && N == 512) {
         // adjoint counterpart: one inverse transform for both rates, two forward
         // transforms (p_x y, p_y y) for the next stage; same tile shape
         constexpr int PL = 2, PNT = (N / 8) * PL;
         e = launch_k<k_row_pair_adj<N, PL, PNT, 6>>(LF_KIND_ROW, dim3(N / PL, B), PNT,
                                                     row_pair_smem_bytes<PL>(N), st, a);
-      } else if constexpr (PP && std::is_same<T, float>::value) {
+      } else if constexpr (PP && N >= 512) {
         // other shapes with p planes: row pairs of one component, 128 threads, five blocks per SM
         constexpr int PL = 1024 / N, PNT = (N / 8) * PL;
         e = launch_k<k_row_rows<N, PL, PNT, 5, ADJ, false>>(LF_KIND_ROW, dim3(N / (2 * PL), B * C), PNT,
                                                             row_rows_smem_bytes<N, PL>(false), st, a);
       } else {
-        e = launch_k<k_row<T, N, C, ADJ, false, RL, RNT, false, RMB>>(LF_KIND_ROW, grow, RNT, smem_row, st, a);
+        e = launch_k<k_row<T, N, C, ADJ, false, RL, RNT, false, RMB, PP>>(LF_KIND_ROW, grow, RNT, smem_row, st, a);
       }
       if (e != cudaSuccess) return e;
     }
@@ -388,36 +388,55 @@ cudaError_t run_lens_pp(const StageArgs& base, int B, int nsteps, double t0, dou
   return cudaSuccess;
 }
 
-// A cluster launch of ``kernel`` on ``clusters`` clusters of CL blocks.
+// A launch of ``Kernel`` on clusters of CL blocks.
+template <auto Kernel, int CL> struct ClusterLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  ClusterLaunch(long clusters, int nt, size_t smem, cudaStream_t st) {
+    cfg.gridDim = dim3((unsigned)(clusters * CL));
+    cfg.blockDim = dim3(nt);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CL;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    // balanced placement up to 128^2: 64 TQU maps 520 -> 493 us, few maps unchanged (256^2: the lens of 48 QU maps
+    // 1,044 -> 1,037 us, but the gradient of 16 TQU maps 2,656 -> 2,718)
+    attr[1].id = cudaLaunchAttributeClusterSchedulingPolicyPreference;
+    attr[1].val.clusterSchedulingPolicyPreference = cudaClusterSchedulingPolicyLoadBalancing;
+    cfg.attrs = attr;
+    cfg.numAttrs = CL <= 8 ? 2 : 1;
+  }
+};
+
 template <auto Kernel, int CL, typename... Args>
 cudaError_t launch_clusters(long clusters, int nt, size_t smem, cudaStream_t st, Args... args) {
   cudaError_t e = ensure_smem<Kernel>(smem, CL > 8);
   if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(clusters * CL));
-  cfg.blockDim = dim3(nt);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CL;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  // balanced placement up to 128^2: 64 TQU maps 520 -> 493 us, few maps unchanged (256^2: the lens of 48 QU maps
-  // 1,044 -> 1,037 us, but the gradient of 16 TQU maps 2,656 -> 2,718)
-  attr[1].id = cudaLaunchAttributeClusterSchedulingPolicyPreference;
-  attr[1].val.clusterSchedulingPolicyPreference = cudaClusterSchedulingPolicyLoadBalancing;
-  cfg.attrs = attr;
-  cfg.numAttrs = CL <= 8 ? 2 : 1;
+  ClusterLaunch<Kernel, CL> l(clusters, nt, smem, st);
   Prof* pf = (g_prof && g_prof->on) ? g_prof : nullptr;
   cudaEvent_t e0 = pf ? pf->next() : nullptr, e1 = pf ? pf->next() : nullptr;
   if (e0) cudaEventRecord(e0, st);
-  e = cudaLaunchKernelEx(&cfg, Kernel, args...);
+  e = cudaLaunchKernelEx(&l.cfg, Kernel, args...);
   if (e1) {
     cudaEventRecord(e1, st);
     pf->kind.push_back(LF_KIND_ROW);
   }
   return e;
+}
+
+// Whether the SMs that ``st`` may use hold a cluster of the kernel.  A process or stream restricted to some of them
+// (a partition of the GPU, a green context) may have no place for one, 16 blocks above all; the lens then takes a
+// launch per stage.  Asked at every call (0.17 us; also while the stream is capturing), since it depends on the stream.
+template <auto Kernel, int CL> bool clusters_fit(int nt, size_t smem, cudaStream_t st) {
+  if (ensure_smem<Kernel>(smem, CL > 8) != cudaSuccess) return false;
+  ClusterLaunch<Kernel, CL> l(1, nt, smem, st);
+  l.cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, Kernel, &l.cfg) == cudaSuccess) return n > 0;
+  cudaGetLastError();
+  return false;
 }
 
 template <typename T, int N, int CL> constexpr size_t cluster_smem() {  // + three mbarriers
@@ -474,6 +493,15 @@ cudaError_t run_store_field(const void* src, void* dst, int dst_f64, long n, cud
   return launch_k<k_store_field<T>>(LF_KIND_ROW, dim3(g), 256, 0, st, static_cast<const T*>(src), dst, dst_f64, n);
 }
 
+template <typename T, int N, bool ADJ, bool PP>
+constexpr auto cluster_lens_kernel = k_lens_cluster<T, N, cluster_blocks<N>(), ADJ, PP, cluster_minb<T, N>()>;
+template <typename T, int N>
+constexpr auto cluster_step_kernel = k_vjp_step_cluster<T, N, cluster_blocks<N>(), cluster_minb<T, N>()>;
+template <typename T, int N, auto Kernel> bool cluster_kernel_fits(cudaStream_t st) {
+  constexpr int CL = cluster_blocks<N>();
+  return clusters_fit<Kernel, CL>(ClGeo<T, N, CL>::NT, cluster_smem<T, N, CL>(), st);
+}
+
 // ``spare``: room for the fields in T; an output that other clusters' inputs share memory with goes there first.
 template <typename T, int N, bool ADJ, bool PP>
 cudaError_t run_lens_cluster(const StageArgs& a, int B, int C, int nsteps, double t0, double t1, void* spare,
@@ -490,7 +518,7 @@ cudaError_t run_lens_cluster(const StageArgs& a, int B, int C, int nsteps, doubl
     c.f_out = spare;
     c.out_f64 = std::is_same<T, double>::value;
   }
-  cudaError_t e = launch_clusters<k_lens_cluster<T, N, CL, ADJ, PP, cluster_minb<T, N>()>, CL>(
+  cudaError_t e = launch_clusters<cluster_lens_kernel<T, N, ADJ, PP>, CL>(
       (long)B * C, ClGeo<T, N, CL>::NT, cluster_smem<T, N, CL>(), st, c);
   if (e != cudaSuccess || !staged) return e;
   return run_store_field<T>(spare, a.f_out, a.out_f64, (long)n, st);
@@ -503,7 +531,6 @@ template <typename T, int N, int C>
 cudaError_t run_vjp_step_cluster(ClusterArgs f, ClusterArgs d, void* pp, const void* phi, double* dacc, int B, int flip,
                                  bool first, cudaStream_t st) {
   constexpr int CL = cluster_blocks<N>();
-  constexpr auto kernel = k_vjp_step_cluster<T, N, CL, cluster_minb<T, N>()>;
   const long P = (long)N * N;
   cudaError_t e = cudaSuccess;
   if constexpr (std::is_same<T, float>::value) {
@@ -517,7 +544,8 @@ cudaError_t run_vjp_step_cluster(ClusterArgs f, ClusterArgs d, void* pp, const v
     e = run_p_planes<T>(a, N, B, 1, f.t0, f.h, st);
     if (e != cudaSuccess) return e;
   }
-  e = launch_clusters<kernel, CL>(2 * f.planes, ClGeo<T, N, CL>::NT, cluster_smem<T, N, CL>(), st, f, d);
+  e = launch_clusters<cluster_step_kernel<T, N>, CL>(2 * f.planes, ClGeo<T, N, CL>::NT, cluster_smem<T, N, CL>(), st,
+                                                     f, d);
   if (e != cudaSuccess) return e;
   const int g = (int)std::min<long>(((long)B * P / 2 + 255) / 256, 148L * 8);
   auto run_dphi = [&](auto minb) {
@@ -527,24 +555,25 @@ cudaError_t run_vjp_step_cluster(ClusterArgs f, ClusterArgs d, void* pp, const v
   return g >= 148 * 6 ? run_dphi(std::integral_constant<int, 3>()) : run_dphi(std::integral_constant<int, 2>());
 }
 
-// The p-plane path (a.pp set) is built for float32 plans, and for float64 ones of N <= 256.
+// N <= 256: clusters where they fit.  Otherwise a launch per row and column pass; p planes (a.pp set) there for
+// float32 plans only.
 template <typename T, int N, int C, bool ADJ>
 cudaError_t run_lens_n(const StageArgs& a, int B, int nsteps, double t0, double t1, cudaStream_t st, bool pp_given) {
   if constexpr (N <= 256) {
-    if (a.pp) {
+    if (a.pp && cluster_kernel_fits<T, N, cluster_lens_kernel<T, N, ADJ, true>>(st)) {
       if (!pp_given) {
         cudaError_t e = run_p_planes<T>(a, N, B, nsteps, 0.0, 1.0 / nsteps, st);
         if (e != cudaSuccess) return e;
       }
       return run_lens_cluster<T, N, ADJ, true>(a, B, C, nsteps, t0, t1, a.y0, st);
     }
-    return run_lens_cluster<T, N, ADJ, false>(a, B, C, nsteps, t0, t1, a.y0, st);
-  } else if constexpr (std::is_same<T, float>::value) {
-    if (a.pp) return run_lens_pp<T, N, C, ADJ, true>(a, B, nsteps, t0, t1, st, pp_given);
-    return run_lens_pp<T, N, C, ADJ, false>(a, B, nsteps, t0, t1, st);
-  } else {
-    return run_lens_pp<T, N, C, ADJ, false>(a, B, nsteps, t0, t1, st);
+    if (!a.pp && cluster_kernel_fits<T, N, cluster_lens_kernel<T, N, ADJ, false>>(st))
+      return run_lens_cluster<T, N, ADJ, false>(a, B, C, nsteps, t0, t1, a.y0, st);
   }
+  if constexpr (std::is_same<T, float>::value) {
+    if (a.pp) return run_lens_pp<T, N, C, ADJ, true>(a, B, nsteps, t0, t1, st, pp_given);
+  }
+  return run_lens_pp<T, N, C, ADJ, false>(a, B, nsteps, t0, t1, st);
 }
 
 template <typename T, int N>
@@ -737,6 +766,53 @@ struct VjpLayout {
   }
 };
 
+// The reverse pass on clusters: one launch and one accumulation per step.  The records of a step's four stages take
+// the twelve planes per component of the two systems, their gradients and stage input in the workspace.
+template <typename T, int N, int C>
+cudaError_t run_vjp_cluster(const StageArgs& af0, const StageArgs& ad0, double* dacc, int B, int nsteps, double t0,
+                            double t1, cudaStream_t st) {
+  const long P = (long)N * N;
+  const double h = (t1 - t0) / nsteps;
+  const size_t plane = sizeof(T) * (size_t)B * C * P;
+  constexpr int io64 = std::is_same<T, double>::value;
+  ClusterArgs f = cluster_args(af0, B, C, 1, t0, h), d = cluster_args(ad0, B, C, 1, t0, h);
+  f.save = af0.y0;
+  d.save = static_cast<char*>(af0.y0) + 8 * plane;
+  void* pp = static_cast<char*>(ad0.between) + plane;
+  // A caller's output that shares memory with what the last step still reads leaves it through the buffers
+  // between the steps: the other system's input (or, not in place, its own) in a single step, the
+  // derivative planes always.
+  const size_t n = (size_t)B * C * P;
+  auto staged = [&](const StageArgs& o) {
+    return (nsteps == 1 && (clobbers(o.f_out, o.out_f64, o.f_in, o.in_f64, n) ||
+                            overlap(o.f_out, n * (o.out_f64 ? 8 : 4), (&o == &af0 ? ad0 : af0).f_in,
+                                    n * (o.in_f64 ? 8 : 4)))) ||
+           overlap(o.f_out, n * (o.out_f64 ? 8 : 4), af0.phi, sizeof(T) * 5 * (size_t)B * P);
+  };
+  const bool want_f = af0.f_out != af0.between, stage_f = want_f && staged(af0), stage_d = staged(ad0);
+  for (int i = 0; i < nsteps; ++i) {
+    const bool last = i == nsteps - 1;
+    f.t0 = d.t0 = t0 + i * h;
+    if (i > 0) {
+      f.f_in = af0.between;
+      d.f_in = ad0.between;
+      f.in_f64 = d.in_f64 = io64;
+    }
+    const bool to_f = last && !stage_f, to_d = last && !stage_d;
+    f.f_out = !to_f ? af0.between : want_f ? af0.f_out : nullptr;
+    d.f_out = !to_d ? ad0.between : ad0.f_out;
+    f.out_f64 = to_f ? af0.out_f64 : io64;
+    d.out_f64 = to_d ? ad0.out_f64 : io64;
+    cudaError_t e = run_vjp_step_cluster<T, N, C>(f, d, pp, af0.phi, dacc, B, 0, i == 0, st);
+    if (e != cudaSuccess) return e;
+  }
+  if (stage_f) {
+    cudaError_t e = run_store_field<T>(af0.between, af0.f_out, af0.out_f64, (long)n, st);
+    if (e != cudaSuccess) return e;
+  }
+  return stage_d ? run_store_field<T>(ad0.between, ad0.f_out, ad0.out_f64, (long)n, st) : cudaSuccess;
+}
+
 template <typename T, int N, int C>
 cudaError_t run_vjp_n(const StageArgs& af0, const StageArgs& ad0, double* dacc, int B, int nsteps, double t0,
                       double t1, cudaStream_t st) {
@@ -751,47 +827,9 @@ cudaError_t run_vjp_n(const StageArgs& af0, const StageArgs& ad0, double* dacc, 
   StageArgs af = af0, ad = ad0;
   const double h = (t1 - t0) / nsteps;
   if constexpr (N <= 256) {
-    // One cluster launch and one accumulation per step.  The records of a step's four stages take the twelve
-    // planes per component of the two systems, their gradients and stage input in the workspace.
-    const size_t plane = sizeof(T) * (size_t)B * C * P;
-    constexpr int io64 = std::is_same<T, double>::value;
-    ClusterArgs f = cluster_args(af0, B, C, 1, t0, h), d = cluster_args(ad0, B, C, 1, t0, h);
-    f.save = af0.y0;
-    d.save = static_cast<char*>(af0.y0) + 8 * plane;
-    void* pp = static_cast<char*>(ad0.between) + plane;
-    // A caller's output that shares memory with what the last step still reads leaves it through the buffers
-    // between the steps: the other system's input (or, not in place, its own) in a single step, the
-    // derivative planes always.
-    const size_t n = (size_t)B * C * P;
-    auto staged = [&](const StageArgs& o) {
-      return (nsteps == 1 && (clobbers(o.f_out, o.out_f64, o.f_in, o.in_f64, n) ||
-                              overlap(o.f_out, n * (o.out_f64 ? 8 : 4), (&o == &af0 ? ad0 : af0).f_in,
-                                      n * (o.in_f64 ? 8 : 4)))) ||
-             overlap(o.f_out, n * (o.out_f64 ? 8 : 4), af0.phi, sizeof(T) * 5 * (size_t)B * P);
-    };
-    const bool want_f = af0.f_out != af0.between, stage_f = want_f && staged(af0), stage_d = staged(ad0);
-    for (int i = 0; i < nsteps; ++i) {
-      const bool last = i == nsteps - 1;
-      f.t0 = d.t0 = t0 + i * h;
-      if (i > 0) {
-        f.f_in = af0.between;
-        d.f_in = ad0.between;
-        f.in_f64 = d.in_f64 = io64;
-      }
-      const bool to_f = last && !stage_f, to_d = last && !stage_d;
-      f.f_out = !to_f ? af0.between : want_f ? af0.f_out : nullptr;
-      d.f_out = !to_d ? ad0.between : ad0.f_out;
-      f.out_f64 = to_f ? af0.out_f64 : io64;
-      d.out_f64 = to_d ? ad0.out_f64 : io64;
-      cudaError_t e = run_vjp_step_cluster<T, N, C>(f, d, pp, af0.phi, dacc, B, 0, i == 0, st);
-      if (e != cudaSuccess) return e;
-    }
-    if (stage_f) {
-      cudaError_t e = run_store_field<T>(af0.between, af0.f_out, af0.out_f64, (long)n, st);
-      if (e != cudaSuccess) return e;
-    }
-    return stage_d ? run_store_field<T>(ad0.between, ad0.f_out, ad0.out_f64, (long)n, st) : cudaSuccess;
-  } else {
+    if (cluster_kernel_fits<T, N, cluster_step_kernel<T, N>>(st))
+      return run_vjp_cluster<T, N, C>(af0, ad0, dacc, B, nsteps, t0, t1, st);
+  }
   const double hh = h / 2.0;
   const double cw[4] = {1.0, 2.0, 2.0, 1.0};
   af.h = ad.h = h;
@@ -826,7 +864,6 @@ cudaError_t run_vjp_n(const StageArgs& af0, const StageArgs& ad0, double* dacc, 
     }
   }
   return cudaSuccess;
-  }
 }
 
 template <typename T, int N>
@@ -871,6 +908,54 @@ struct CkptLayout {
   }
 };
 
+// The checkpointed pass (run_vjp_ckpt_n) on clusters: the forward lens with its checkpoints, then the launches per
+// step of run_vjp_cluster.
+template <typename T, int N, int C>
+cudaError_t run_vjp_ckpt_cluster(const StageArgs& af0, const StageArgs& ad0, char* ckpt, char* grads, void* sink,
+                                 double* dacc, int B, int nsteps, double t0, double t1, cudaStream_t st) {
+  const long P = (long)N * N;
+  const size_t plane = sizeof(T) * (size_t)B * C * P;
+  const double h = (t1 - t0) / nsteps, hb = -h;  // the adjoint integration runs t1 -> t0
+  StageArgs af = af0;
+  cudaError_t e;
+  constexpr int io64 = std::is_same<T, double>::value;
+  if (af.f_out == sink) af.f_out = nullptr;
+  // the p planes of the forward lens, if they fit what the reverse steps use later
+  if ((size_t)((char*)dacc - (char*)af.y0) >= sizeof(T) * 2 * (2 * (size_t)nsteps + 1) * P * B) {
+    af.pp = af.y0;
+    e = run_p_planes<T>(af, N, B, nsteps, 0.0, 1.0 / nsteps, st);
+    if (e != cudaSuccess) return e;
+    e = run_lens_cluster<T, N, false, true>(af, B, C, nsteps, t0, t1, sink, st, ckpt);
+  } else {
+    e = run_lens_cluster<T, N, false, false>(af, B, C, nsteps, t0, t1, sink, st, ckpt);
+  }
+  if (e != cudaSuccess) return e;
+  ClusterArgs f = cluster_args(af0, B, C, 1, t0, h), d = cluster_args(ad0, B, C, 1, t1, hb);
+  f.in_f64 = io64;
+  f.f_out = nullptr;
+  f.save = grads;
+  d.save = ad0.y0;
+  const size_t nf = (size_t)B * C * P;
+  const bool stage_d = (nsteps == 1 && clobbers(ad0.f_out, ad0.out_f64, ad0.f_in, ad0.in_f64, nf)) ||
+                       overlap(ad0.f_out, nf * (ad0.out_f64 ? 8 : 4), af0.phi, sizeof(T) * 5 * (size_t)B * P);
+  for (int ib = 0; ib < nsteps; ++ib) {
+    const int i = nsteps - 1 - ib;
+    const bool to_d = ib == nsteps - 1 && !stage_d;
+    f.f_in = ckpt + (size_t)i * plane;
+    f.t0 = t0 + i * h;
+    d.t0 = t0 + (i + 1) * h;
+    if (ib > 0) {
+      d.f_in = ad0.between;
+      d.in_f64 = io64;
+    }
+    d.f_out = to_d ? ad0.f_out : ad0.between;
+    d.out_f64 = to_d ? ad0.out_f64 : io64;
+    e = run_vjp_step_cluster<T, N, C>(f, d, af0.between, af0.phi, dacc, B, 1, ib == 0, st);
+    if (e != cudaSuccess) return e;
+  }
+  return stage_d ? run_store_field<T>(ad0.between, ad0.f_out, ad0.out_f64, (long)nf, st) : cudaSuccess;
+}
+
 // The exact transpose of the discrete forward RK4 (lense_flow.py:336-352 with
 // util.py:184-199).  The forward integration stores y_i at the start of every
 // step.  Backwards, step i is recomputed from y_i with its four stage
@@ -903,44 +988,12 @@ cudaError_t run_vjp_ckpt_n(const StageArgs& af0, const StageArgs& ad0, char* ckp
   const double cw[4] = {1.0, 2.0, 2.0, 1.0};
   StageArgs af = af0, ad = ad0;
   cudaError_t e;
-  if constexpr (N <= 256) {  // as run_vjp_n: the forward lens with its checkpoints, then two launches per step
-    constexpr int io64 = std::is_same<T, double>::value;
-    if (af.f_out == sink) af.f_out = nullptr;
-    // the p planes of the forward lens, if they fit what the reverse steps use later
-    if ((size_t)((char*)dacc - (char*)af.y0) >= sizeof(T) * 2 * (2 * (size_t)nsteps + 1) * P * B) {
-      af.pp = af.y0;
-      e = run_p_planes<T>(af, N, B, nsteps, 0.0, 1.0 / nsteps, st);
-      if (e != cudaSuccess) return e;
-      e = run_lens_cluster<T, N, false, true>(af, B, C, nsteps, t0, t1, sink, st, ckpt);
-    } else {
-      e = run_lens_cluster<T, N, false, false>(af, B, C, nsteps, t0, t1, sink, st, ckpt);
-    }
-    if (e != cudaSuccess) return e;
-    ClusterArgs f = cluster_args(af0, B, C, 1, t0, h), d = cluster_args(ad0, B, C, 1, t1, hb);
-    f.in_f64 = io64;
-    f.f_out = nullptr;
-    f.save = grads;
-    d.save = ad0.y0;
-    const size_t nf = (size_t)B * C * P;
-    const bool stage_d = (nsteps == 1 && clobbers(ad0.f_out, ad0.out_f64, ad0.f_in, ad0.in_f64, nf)) ||
-                         overlap(ad0.f_out, nf * (ad0.out_f64 ? 8 : 4), af0.phi, sizeof(T) * 5 * (size_t)B * P);
-    for (int ib = 0; ib < nsteps; ++ib) {
-      const int i = nsteps - 1 - ib;
-      const bool to_d = ib == nsteps - 1 && !stage_d;
-      f.f_in = ckpt + (size_t)i * plane;
-      f.t0 = t0 + i * h;
-      d.t0 = t0 + (i + 1) * h;
-      if (ib > 0) {
-        d.f_in = ad0.between;
-        d.in_f64 = io64;
-      }
-      d.f_out = to_d ? ad0.f_out : ad0.between;
-      d.out_f64 = to_d ? ad0.out_f64 : io64;
-      e = run_vjp_step_cluster<T, N, C>(f, d, af0.between, af0.phi, dacc, B, 1, ib == 0, st);
-      if (e != cudaSuccess) return e;
-    }
-    return stage_d ? run_store_field<T>(ad0.between, ad0.f_out, ad0.out_f64, (long)nf, st) : cudaSuccess;
-  } else {
+  if constexpr (N <= 256) {
+    if (cluster_kernel_fits<T, N, cluster_step_kernel<T, N>>(st) &&
+        cluster_kernel_fits<T, N, cluster_lens_kernel<T, N, false, true>>(st) &&
+        cluster_kernel_fits<T, N, cluster_lens_kernel<T, N, false, false>>(st))
+      return run_vjp_ckpt_cluster<T, N, C>(af0, ad0, ckpt, grads, sink, dacc, B, nsteps, t0, t1, st);
+  }
   // ---- forward integration, storing y_i at the start of each step
   af.h = h;
   af.stage = 0;
@@ -1019,7 +1072,6 @@ cudaError_t run_vjp_ckpt_n(const StageArgs& af0, const StageArgs& ad0, char* ckp
     }
   }
   return cudaSuccess;
-  }
 }
 
 template <typename T, int N>

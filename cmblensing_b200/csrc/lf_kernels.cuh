@@ -54,7 +54,7 @@ struct StageArgs {
   void* grad;       // standard pass with SAVE: d_x y_s, d_y y_s, [B*C][2][N][N] T
   void* dsave;      // adjoint pass with SAVE: next stage input, [B*C][N][N] T
   void* between;    // reverse pass on clusters (N <= 256): fields between steps, p planes of a step
-  // p = M(t)^-1 grad(phi) at the 2n+1 stage times t0 + k h/2 (row pass with PP):
+  // p = M(t)^-1 grad(phi) at the 2n+1 stage times t0 + k h/2, or null:
   // [B][pp_k][2][N][N] T; this stage reads time index pp_idx
   const void* pp;
   int pp_k;
@@ -290,8 +290,10 @@ __global__ void __launch_bounds__(NT, MINB) k_col(StageArgs a) {
 // STAGE0: initialisation (copy the input field, transform the first stage
 // input), no rate.  SAVE (reverse mode): the standard pass also stores
 // d_x y_s and d_y y_s; the adjoint pass stores its next stage input.
-// p is formed from the five derivative planes; lenses with p planes take the row-pair passes below.
-template <typename T, int N, int C, bool ADJ, bool STAGE0, int LINES, int NT, bool SAVE = false, int MINB = 1>
+// PP: p at the stage time is read from the p planes (N <= 256 where clusters do not fit; larger maps with p planes
+// take the row-pair passes below) instead of being formed from the five derivative planes.
+template <typename T, int N, int C, bool ADJ, bool STAGE0, int LINES, int NT, bool SAVE = false, int MINB = 1,
+          bool PP = false>
 __global__ void __launch_bounds__(NT, MINB) k_row(StageArgs a) {
   constexpr int H = N / 2;
   constexpr long P = (long)N * N;
@@ -378,17 +380,31 @@ __global__ void __launch_bounds__(NT, MINB) k_row(StageArgs a) {
     // p at the rate time (standard) and at the next stage time (adjoint)
     T prx[2][2], pry[2][2];
     if (need_phi) {
-      c2<T> fx[2], fy[2], fxx[2], fxy[2], fyy[2];
-      ld2<T>(reinterpret_cast<const c2<T>*>(phi) + e0, fx);
-      ld2<T>(reinterpret_cast<const c2<T>*>(phi + P) + e0, fy);
-      ld2<T>(reinterpret_cast<const c2<T>*>(phi + 2 * P) + e0, fxx);
-      ld2<T>(reinterpret_cast<const c2<T>*>(phi + 3 * P) + e0, fxy);
-      ld2<T>(reinterpret_cast<const c2<T>*>(phi + 4 * P) + e0, fyy);
-      const T tp = ADJ ? tnext : tcur;
+      if constexpr (PP) {
+        const T* pp = reinterpret_cast<const T*>(a.pp) + (map * a.pp_k + a.pp_idx) * 2 * P + (long)r0 * N;
+        c2<T> px[2], py[2];
+        ld2<T>(reinterpret_cast<const c2<T>*>(pp) + e0, px);
+        ld2<T>(reinterpret_cast<const c2<T>*>(pp + P) + e0, py);
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        p_vector<T>(fx[q].x, fy[q].x, fxx[q].x, fxy[q].x, fyy[q].x, tp, prx[q][0], pry[q][0]);
-        p_vector<T>(fx[q].y, fy[q].y, fxx[q].y, fxy[q].y, fyy[q].y, tp, prx[q][1], pry[q][1]);
+        for (int q = 0; q < 2; ++q) {
+          prx[q][0] = px[q].x;
+          prx[q][1] = px[q].y;
+          pry[q][0] = py[q].x;
+          pry[q][1] = py[q].y;
+        }
+      } else {
+        c2<T> fx[2], fy[2], fxx[2], fxy[2], fyy[2];
+        ld2<T>(reinterpret_cast<const c2<T>*>(phi) + e0, fx);
+        ld2<T>(reinterpret_cast<const c2<T>*>(phi + P) + e0, fy);
+        ld2<T>(reinterpret_cast<const c2<T>*>(phi + 2 * P) + e0, fxx);
+        ld2<T>(reinterpret_cast<const c2<T>*>(phi + 3 * P) + e0, fxy);
+        ld2<T>(reinterpret_cast<const c2<T>*>(phi + 4 * P) + e0, fyy);
+        const T tp = ADJ ? tnext : tcur;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          p_vector<T>(fx[q].x, fy[q].x, fxx[q].x, fxy[q].x, fyy[q].x, tp, prx[q][0], pry[q][0]);
+          p_vector<T>(fx[q].y, fy[q].y, fxx[q].y, fxy[q].y, fyy[q].y, tp, prx[q][1], pry[q][1]);
+        }
       }
     }
 #pragma unroll
