@@ -164,11 +164,14 @@ template <typename T, bool INV> LF_HD void dft8(c2<T>* a) {
 
 // A constant twiddle w = wr + i wi as f (1 + i t), f = wr (``re``), or as f (t + i), f = wi: an equal number of
 // operations, but the rounded f and f t are off by different amounts.  A constant's error is the same in every
-// transform and adds up over the stages of a lens, unlike the roundings of the data, so the form whose constants
-// come out closer is taken, with t the quotient by the rounded f.  Units of 2^-24, nearest f and wi / wr of the
-// larger part -> this: pi/16 0.51 -> 0.04, pi/8 0.49 -> 0.37, 3 pi/16 0.55 -> 0.29.  Relative error of float32
-// lenses, n = 7, against the float64 engine: T 256^2 9.2e-8 -> 8.5e-8, QU 512^2 9.7e-8 -> 9.3e-8, TQU 1024^2
-// 1.09e-7 -> 1.00e-7, adjoint TQU 1024^2 1.25e-7 -> 1.17e-7.
+// transform and adds up over the stages of a lens, unlike the roundings of the data, so in float32 the form whose
+// constants come out closer is taken, with t the quotient by the rounded f.  Units of 2^-24, nearest f and wi / wr of
+// the larger part -> this: pi/16 0.51 -> 0.04, pi/8 0.49 -> 0.37, 3 pi/16 0.55 -> 0.29.  Relative error of i k FFT
+// pairs of white noise (host): L = 256 as 16 x 16 1.44e-7 -> 1.40e-7, 512 as 16 x 32 1.59e-7 -> 1.49e-7, 1024 as
+// 32 x 32 1.78e-7 -> 1.56e-7 (16 x 8 x 8 1.61e-7).
+// LARGER: f the larger part.  For the 16-point halves of a 32-point transform, whose column pass takes half a
+// microsecond more in launches of a few blocks with the other form at pi/8 (reverse pass of one T map of 512^2
+// 1,088 -> 1,119 us), and for float64, whose constants are not rounded again.
 template <typename T> struct TwForm {
   T f, t;
   bool re;
@@ -177,15 +180,16 @@ template <typename T> __host__ __device__ constexpr double tw_error(double f, do
   const double a = double(T(f)), b = a * double(T(g / a));
   return (a - f) * (a - f) + (b - g) * (b - g);
 }
-template <typename T> __host__ __device__ constexpr TwForm<T> tw_form(double wr, double wi) {
-  if (tw_error<T>(wr, wi) <= tw_error<T>(wi, wr)) return TwForm<T>{T(wr), T(wi / double(T(wr))), true};
+template <typename T, bool LARGER = false> __host__ __device__ constexpr TwForm<T> tw_form(double wr, double wi) {
+  const bool re = LARGER || sizeof(T) == 8 ? wr * wr >= wi * wi : tw_error<T>(wr, wi) <= tw_error<T>(wi, wr);
+  if (re) return TwForm<T>{T(wr), T(wi / double(T(wr))), true};
   return TwForm<T>{T(wi), T(wr / double(T(wi))), false};
 }
 
 // a <- a + w b, b <- a - w b for a constant twiddle w = (wr, wi), with FMAs: the scaled b costs two and each
 // output two more (six instructions instead of eight for a multiply, then an add and a subtract).
-template <typename T> LF_HD void bfly_w(c2<T>& a, c2<T>& b, double wr, double wi) {
-  const TwForm<T> w = tw_form<T>(wr, wi);
+template <typename T, bool LARGER = false> LF_HD void bfly_w(c2<T>& a, c2<T>& b, double wr, double wi) {
+  const TwForm<T> w = tw_form<T, LARGER>(wr, wi);
   const c2<T> u = w.re ? mk<T>(b.x - w.t * b.y, b.y + w.t * b.x) : mk<T>(w.t * b.x - b.y, w.t * b.y + b.x);
   const c2<T> a0 = a;
   a = caxpy<T>(w.f, u, a0);
@@ -193,7 +197,7 @@ template <typename T> LF_HD void bfly_w(c2<T>& a, c2<T>& b, double wr, double wi
 }
 
 // Radix-2 split into two 8-point DFTs: X[k] = E[k] + W16^k O[k], X[k+8] = E[k] - W16^k O[k].
-template <typename T, bool INV> LF_HD void dft16(c2<T>* a) {
+template <typename T, bool INV, bool HALF = false> LF_HD void dft16(c2<T>* a) {
   c2<T> e[8], o[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -212,7 +216,7 @@ template <typename T, bool INV> LF_HD void dft16(c2<T>* a) {
       a[k] = cadd<T>(e[k], t);
       a[k + 8] = csub<T>(e[k], t);
     } else {
-      bfly_w<T>(e[k], o[k], wr[k], INV ? ws[k] : -ws[k]);
+      bfly_w<T, HALF>(e[k], o[k], wr[k], INV ? ws[k] : -ws[k]);
       a[k] = e[k];
       a[k + 8] = o[k];
     }
@@ -233,8 +237,8 @@ template <typename T, bool INV> LF_HD void dft32(c2<T>* a) {
     e[i] = a[2 * i];
     o[i] = a[2 * i + 1];
   }
-  dft16<T, INV>(e);
-  dft16<T, INV>(o);
+  dft16<T, INV, true>(e);
+  dft16<T, INV, true>(o);
   // W32^k forward = (cos(pi k/16), -sin(pi k/16)), k = 0..15
   const double wr[16] = {1.0,     LF_C11,  LF_C22,  LF_C33,  LF_C45,  LF_S33,  LF_S22,  LF_S11,
                          0.0,     -LF_S11, -LF_S22, -LF_S33, -LF_C45, -LF_C33, -LF_C22, -LF_C11};
