@@ -426,17 +426,18 @@ cudaError_t launch_clusters(long clusters, int nt, size_t smem, cudaStream_t st,
   return e;
 }
 
-// Whether the SMs that ``st`` may use hold a cluster of the kernel.  A process or stream restricted to some of them
-// (a partition of the GPU, a green context) may have no place for one, 16 blocks above all; the lens then takes a
-// launch per stage.  Asked at every call (0.17 us; also while the stream is capturing), since it depends on the stream.
-template <auto Kernel, int CL> bool clusters_fit(int nt, size_t smem, cudaStream_t st) {
-  if (ensure_smem<Kernel>(smem, CL > 8) != cudaSuccess) return false;
+// Clusters of the kernel that the SMs which ``st`` may use hold at once.  A process or stream restricted to some of
+// them (a partition of the GPU, a green context) may have no place for one, 16 blocks above all; the lens then takes
+// a launch per stage.  Asked at every call (0.17 us; also while the stream is capturing), since it depends on the
+// stream.
+template <auto Kernel, int CL> int resident_clusters(int nt, size_t smem, cudaStream_t st) {
+  if (ensure_smem<Kernel>(smem, CL > 8) != cudaSuccess) return 0;
   ClusterLaunch<Kernel, CL> l(1, nt, smem, st);
   l.cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, Kernel, &l.cfg) == cudaSuccess) return n > 0;
+  if (cudaOccupancyMaxActiveClusters(&n, Kernel, &l.cfg) == cudaSuccess) return n;
   cudaGetLastError();
-  return false;
+  return 0;
 }
 
 template <typename T, int N, int CL> constexpr size_t cluster_smem() {  // + three mbarriers
@@ -497,9 +498,9 @@ template <typename T, int N, bool ADJ, bool PP>
 constexpr auto cluster_lens_kernel = k_lens_cluster<T, N, cluster_blocks<N>(), ADJ, PP, cluster_minb<T, N>()>;
 template <typename T, int N>
 constexpr auto cluster_step_kernel = k_vjp_step_cluster<T, N, cluster_blocks<N>(), cluster_minb<T, N>()>;
-template <typename T, int N, auto Kernel> bool cluster_kernel_fits(cudaStream_t st) {
+template <typename T, int N, auto Kernel> int resident(cudaStream_t st) {
   constexpr int CL = cluster_blocks<N>();
-  return clusters_fit<Kernel, CL>(ClGeo<T, N, CL>::NT, cluster_smem<T, N, CL>(), st);
+  return resident_clusters<Kernel, CL>(ClGeo<T, N, CL>::NT, cluster_smem<T, N, CL>(), st);
 }
 
 // ``spare``: room for the fields in T; an output that other clusters' inputs share memory with goes there first.
@@ -560,15 +561,25 @@ cudaError_t run_vjp_step_cluster(ClusterArgs f, ClusterArgs d, void* pp, const v
 template <typename T, int N, int C, bool ADJ>
 cudaError_t run_lens_n(const StageArgs& a, int B, int nsteps, double t0, double t1, cudaStream_t st, bool pp_given) {
   if constexpr (N <= 256) {
-    if (a.pp && cluster_kernel_fits<T, N, cluster_lens_kernel<T, N, ADJ, true>>(st)) {
+    if (a.pp && resident<T, N, cluster_lens_kernel<T, N, ADJ, true>>(st)) {
       if (!pp_given) {
         cudaError_t e = run_p_planes<T>(a, N, B, nsteps, 0.0, 1.0 / nsteps, st);
         if (e != cudaSuccess) return e;
       }
       return run_lens_cluster<T, N, ADJ, true>(a, B, C, nsteps, t0, t1, a.y0, st);
     }
-    if (!a.pp && cluster_kernel_fits<T, N, cluster_lens_kernel<T, N, ADJ, false>>(st))
-      return run_lens_cluster<T, N, ADJ, false>(a, B, C, nsteps, t0, t1, a.y0, st);
+    // p formed from the derivative planes costs a cluster almost a stage, once per component plane; the row pass
+    // forms it once per map.  256^2 QU, us per lens of n = 7 in passes and on clusters (14 at once), 24, 30, 64, 128
+    // and 192 planes: 520, 670, 1,101, 2,041, 3,049 and 496, 712, 1,246, 2,469, 3,555; adjoint 48, 64, 128 planes:
+    // 1,022, 1,227, 2,303 and 1,000, 1,291, 2,570.  T and TQU maps: within 5% of one another there.
+    auto passes_faster = [&](int clusters) {
+      return N == 256 && C == 2 && sizeof(T) == 4 && (long)B * C > (ADJ ? 4 : 2) * (long)clusters;
+    };
+    if (!a.pp) {
+      const int clusters = resident<T, N, cluster_lens_kernel<T, N, ADJ, false>>(st);
+      if (clusters && !passes_faster(clusters))
+        return run_lens_cluster<T, N, ADJ, false>(a, B, C, nsteps, t0, t1, a.y0, st);
+    }
   }
   if constexpr (std::is_same<T, float>::value) {
     if (a.pp) return run_lens_pp<T, N, C, ADJ, true>(a, B, nsteps, t0, t1, st, pp_given);
@@ -827,8 +838,13 @@ cudaError_t run_vjp_n(const StageArgs& af0, const StageArgs& ad0, double* dacc, 
   StageArgs af = af0, ad = ad0;
   const double h = (t1 - t0) / nsteps;
   if constexpr (N <= 256) {
-    if (cluster_kernel_fits<T, N, cluster_step_kernel<T, N>>(st))
-      return run_vjp_cluster<T, N, C>(af0, ad0, dacc, B, nsteps, t0, t1, st);
+    // Many float64 maps of 256^2 in two or three components keep the row passes' shared p faster than seven clusters
+    // at once.  ms in passes and on clusters, n = 7: QU, 64, 96, 192 planes 7.5, 10.9, 20.4 and 7.5, 11.1, 21.8; TQU,
+    // 45, 60, 96, 144 planes 5.3, 6.6, 9.7, 14.1 and 5.2, 6.8, 10.7, 15.9.
+    const int clusters = resident<T, N, cluster_step_kernel<T, N>>(st);
+    const bool passes_faster =
+        N == 256 && sizeof(T) == 8 && C >= 2 && (long)B * C > (C == 2 ? 12 : 8) * (long)clusters;
+    if (clusters && !passes_faster) return run_vjp_cluster<T, N, C>(af0, ad0, dacc, B, nsteps, t0, t1, st);
   }
   const double hh = h / 2.0;
   const double cw[4] = {1.0, 2.0, 2.0, 1.0};
@@ -989,9 +1005,8 @@ cudaError_t run_vjp_ckpt_n(const StageArgs& af0, const StageArgs& ad0, char* ckp
   StageArgs af = af0, ad = ad0;
   cudaError_t e;
   if constexpr (N <= 256) {
-    if (cluster_kernel_fits<T, N, cluster_step_kernel<T, N>>(st) &&
-        cluster_kernel_fits<T, N, cluster_lens_kernel<T, N, false, true>>(st) &&
-        cluster_kernel_fits<T, N, cluster_lens_kernel<T, N, false, false>>(st))
+    if (resident<T, N, cluster_step_kernel<T, N>>(st) && resident<T, N, cluster_lens_kernel<T, N, false, true>>(st) &&
+        resident<T, N, cluster_lens_kernel<T, N, false, false>>(st))
       return run_vjp_ckpt_cluster<T, N, C>(af0, ad0, ckpt, grads, sink, dacc, B, nsteps, t0, t1, st);
   }
   // ---- forward integration, storing y_i at the start of each step
