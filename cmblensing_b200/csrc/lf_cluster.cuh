@@ -5,7 +5,8 @@
 // [r KC, (r+1) KC) of the row spectra; the RK4 state (y0, acc) stays in
 // registers, the row spectra in shared memory, and the two transpositions of
 // a stage (rows -> columns before the column pass, back after it) are stores
-// into the other blocks' shared memory, each followed by a cluster barrier.
+// into the other blocks' shared memory, counted on the receiving block's
+// mbarriers; a stage has no barrier of the cluster or of a block.
 // Per stage HBM/L2 sees only the p planes.
 //
 // A group of TP = N / E lanes of one warp holds a length-N transform, E
@@ -38,7 +39,7 @@ template <typename T, int N, int CL> struct ClGeo {
   static constexpr int RPC = 2 * G;      // rows per block
   static constexpr int KC = G;           // packed columns per block
   static_assert(N == 64 || N == 128 || N == 256, "a group is at most one warp");
-  static_assert(NT % 32 == 0 && KC >= 8, "whole warps, 64-byte pushes");
+  static_assert(NT % 32 == 0 && CL > 1 && KC == 8, "whole warps, several blocks, 64-byte puts");
 };
 
 // Radices of the length-N group transform in forward order (the inverse runs them reversed): one pass of
@@ -84,7 +85,7 @@ template <typename T, int N> __host__ __device__ constexpr int lay_step() {
 template <typename T, int N> __host__ __device__ constexpr int lay_group() {
   return sizeof(T) == 4 && N == 64 ? 184 : lay_step<T, N>() + lay_size<T, N>();
 }
-constexpr int log2_of(int n) { return n <= 1 ? 0 : 1 + log2_of(n / 2); }
+__host__ __device__ constexpr int log2_of(int n) { return n <= 1 ? 0 : 1 + log2_of(n / 2); }
 
 // A row transform in one row's scratch.
 template <typename T, int N> struct RowLay {
@@ -112,7 +113,7 @@ template <typename T, int N> struct ColLay {
 // bank conflicts.  Groups of sixteen lanes or more see those bits in the lane alone; with eight lanes
 // (float32, N = 64) two groups share 128 bytes, one line (two rows) apart.
 template <typename T, int N, int KC> __host__ __device__ __forceinline__ constexpr int col_at(int m, int line) {
-  return m * KC + (line ^ (sizeof(T) == 8 ? m & 7 : N == 64 ? (KC == 8 ? m & 6 : (m & 7) << 1) : KC == 8 ? (m >> 1) & 7 : m & 15));
+  return m * KC + (line ^ (sizeof(T) == 8 ? m & 7 : N == 64 ? m & 6 : (m >> 1) & 7));
 }
 template <typename T, int N, int RPC> __host__ __device__ __forceinline__ constexpr int land_at(int k, int row) {
   return k * RPC + (row ^ (sizeof(T) == 8 ? k & 7 : N == 64 ? (k & 1) | ((k & 6) << 1) : k & 15));
@@ -161,23 +162,15 @@ __device__ __forceinline__ bool cluster_mbar_wait(uint64_t* mbar, uint32_t parit
   }
   return false;
 }
-template <int CL> __device__ __forceinline__ void cluster_sync() {
-  if constexpr (CL > 1) {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  } else {
-    __syncthreads();
-  }
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-
 // The way out of a warp whose wait ran out.  The cluster's other warps miss its puts, so that their own next wait
 // runs out too: each waits once more at most (about two seconds with its drain), puts nothing after that and comes
 // here or has finished.  The barrier, which threads that have exited do not hold up, keeps every block's shared
 // memory until the last put into it has been sent and drained.
-__device__ __forceinline__ void cluster_leave() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void cluster_leave() { cluster_sync(); }
 
 // ------------------------------------------------------ group transforms
 // One radix-R pass on registers: butterfly i of a lane is b = lane + TP i, its input r in register i + (E/R) r.
@@ -304,33 +297,26 @@ template <typename T, int N, int CL> struct ClSystem {
 
   // one thread, before the first cluster_sync
   __device__ __forceinline__ void init_barriers() const {
-    if constexpr (CL > 1) {
-      for (int i = 0; i < 2; ++i) {
-        mbar_init(mbar + i, 1);
-        mbar_expect_tx(mbar + i, kPhaseBytes);
-      }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(mbar + i, 1);
+      mbar_expect_tx(mbar + i, kPhaseBytes);
     }
   }
   // All of area ``which`` has landed for phase number ``phase``; ``more``: another phase follows.  False, for the
   // whole warp, if a lane's wait ran out: recorded, then drained like wait_or_record, and the warp leaves by
   // cluster_leave.
   __device__ __forceinline__ bool landed(int which, int phase, int polls, bool more) const {
-    if constexpr (CL > 1) {
-      const bool ok = cluster_mbar_wait(mbar + which, phase & 1, polls);
-      if (!ok) {
-        record_timeout();
-        cluster_mbar_wait(mbar + which, phase & 1, kWaitTries);
-      }
-      if (!__all_sync(0xffffffffu, ok)) return false;
-      if (threadIdx.x == 0 && more) mbar_expect_tx(mbar + which, kPhaseBytes);
-    } else {
-      __syncthreads();
+    const bool ok = cluster_mbar_wait(mbar + which, phase & 1, polls);
+    if (!ok) {
+      record_timeout();
+      cluster_mbar_wait(mbar + which, phase & 1, kWaitTries);
     }
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    if (threadIdx.x == 0 && more) mbar_expect_tx(mbar + which, kPhaseBytes);
     return true;
   }
   __device__ __forceinline__ void put(c2<T>* local, uint32_t to, int which, c2<T> v) const {
-    if constexpr (CL == 1) *local = v;
-    else cluster_put(cluster_addr(smem_addr(local), to), cluster_addr(smem_addr(mbar + which), to), v);
+    cluster_put(cluster_addr(smem_addr(local), to), cluster_addr(smem_addr(mbar + which), to), v);
   }
 
   // Column phase: Gx = IFFT(i KX / N^2 FFT(S)) of column g, to the blocks that own its rows.  ``before`` runs
@@ -538,7 +524,7 @@ __device__ __forceinline__ void cl_integrate(const ClusterArgs& a, long cmap) {
   static_assert(S::kElems * sizeof(c2<T>) % 16 == 0, "the table is copied to a 16-byte boundary");
   static_assert(TW * sizeof(c2<T>) % 16 == 0, "twiddle table: one bulk copy");
   const int tid = threadIdx.x;
-  const uint32_t rank = CL > 1 ? cluster_rank() : 0u;
+  const uint32_t rank = cluster_rank();
   const long map = cmap / a.ncomp;
   S sys;
   sys.init(data, mbar + 1, tw, tid, rank);
@@ -601,7 +587,7 @@ __device__ __forceinline__ void cl_integrate(const ClusterArgs& a, long cmap) {
     }
   int k_now = -1;
   if constexpr (SAVE && ADJ) store(save, y0);
-  cluster_sync<CL>();       // every block runs, with its barriers initialised, before anyone puts into it
+  cluster_sync();           // every block runs, with its barriers initialised, before anyone puts into it
   wait_or_record(mbar, 0);  // (a timed-out wait is recorded; the block goes on to its next wait)
   if constexpr (ADJ) {
     load_p(0);

@@ -39,7 +39,7 @@ struct StageArgs {
   void* gx;  // column pass output
   const void* twN;  // N complex T, exp(-2 pi i k / N)
   const void* twP;  // pass table of length N (ptw_size(N) complex T): column pass, paired row pass
-  const void* twC;  // column table of the two-pass column plan (ctw_size(N) complex T; N = 512)
+  const void* twC;  // column table of the two-pass column plan (ctw_size(N) complex T; N = 512, 1024)
   const void* twR;  // table of the row-pair passes (rtw_size(N) complex T; N = 512, 1024)
   const void* twG;  // table of the cluster kernels' group transforms (N <= 256)
   double kbase;     // 2 pi / (N d)
@@ -991,7 +991,8 @@ __global__ void __launch_bounds__(NT, MINB) k_row_rows(StageArgs a) {
   const c2<T>* tw3 = tw + (RM - 1) * 8;       // (8, N / 8)
   const T ky_scale = T(a.kbase / double(N));
   __syncthreads();  // barriers initialised before anyone waits on them
-  // a timed-out wait is recorded and the block goes on, so that every thread meets every barrier below
+  // a timed-out wait is recorded and the block goes on; at the staged operands' wait below its threads leave, which
+  // no barrier waits for
   wait_or_record(mbar + 1, 0);
 
   c2<T> w[2][R];
