@@ -936,14 +936,15 @@ cudaError_t run_vjp_ckpt_cluster(const StageArgs& af0, const StageArgs& ad0, cha
   cudaError_t e;
   constexpr int io64 = std::is_same<T, double>::value;
   if (af.f_out == sink) af.f_out = nullptr;
+  void* spare = af0.between;  // where the p planes of a step go later
   // the p planes of the forward lens, if they fit what the reverse steps use later
   if ((size_t)((char*)dacc - (char*)af.y0) >= sizeof(T) * 2 * (2 * (size_t)nsteps + 1) * P * B) {
     af.pp = af.y0;
     e = run_p_planes<T>(af, N, B, nsteps, 0.0, 1.0 / nsteps, st);
     if (e != cudaSuccess) return e;
-    e = run_lens_cluster<T, N, false, true>(af, B, C, nsteps, t0, t1, sink, st, ckpt);
+    e = run_lens_cluster<T, N, false, true>(af, B, C, nsteps, t0, t1, spare, st, ckpt);
   } else {
-    e = run_lens_cluster<T, N, false, false>(af, B, C, nsteps, t0, t1, sink, st, ckpt);
+    e = run_lens_cluster<T, N, false, false>(af, B, C, nsteps, t0, t1, spare, st, ckpt);
   }
   if (e != cudaSuccess) return e;
   ClusterArgs f = cluster_args(af0, B, C, 1, t0, h), d = cluster_args(ad0, B, C, 1, t1, hb);

@@ -151,3 +151,24 @@ def test_reverse_pass_outputs_over_inputs(torch_cuda, N, B, io64, case, n):
     assert torch.equal(out, want) and torch.equal(dphi, want_dphi)
     if back is not None:
         assert torch.equal(back, other)
+
+
+@pytest.mark.parametrize("n", [3, 9])
+def test_checkpointed_pass_with_a_shifted_lensed_field(torch_cuda, n):
+    """The lensed field one map behind the input, with step counts whose p planes end before and in the last of the
+    workspace's regions that the forward lens may use."""
+    torch = torch_cuda
+    from cmblensing_b200 import _native as nat
+    N, B, C = 256, 20, 2
+    plan, f, phi = _problem(torch, N, B, C)
+    f = f.float()
+    cot = f.flip(0).contiguous()
+    planes = plan.phi_planes(phi)
+    dphi = torch.empty((B, N, N // 2 + 1), dtype=torch.complex128, device="cuda")
+    want, lensed, want_dphi = torch.empty_like(f), torch.empty_like(f), torch.empty_like(dphi)
+    _reverse(torch, "exact", plan, B, n, f, cot, planes, want, lensed, want_dphi, nat.LF_F32)
+    buf = torch.empty((B + 1, C, N, N), dtype=torch.float32, device="cuda")
+    buf[:B] = f
+    out = torch.empty_like(f)
+    _reverse(torch, "exact", plan, B, n, buf[:B], cot, planes, out, buf[1:], dphi, nat.LF_F32)
+    assert torch.equal(buf[1:], lensed) and torch.equal(out, want) and torch.equal(dphi, want_dphi)
