@@ -288,13 +288,13 @@ cudaError_t launch_col(int planes, cudaStream_t st, const StageArgs& a) {
   }
 }
 
-// p = M(t)^-1 grad(phi) at the 2n+1 times t0 + k h / 2 from the derivative planes
+// p = M(t)^-1 grad(phi) at the 2n+1 times t0 + (k0 + k) h / 2 from the derivative planes
 template <typename T>
-cudaError_t run_p_planes(const StageArgs& a, int N, int B, int nsteps, double t0, double h, cudaStream_t st) {
+cudaError_t run_p_planes(const StageArgs& a, int N, int B, int nsteps, double t0, double h, cudaStream_t st, int k0 = 0) {
   const long P = (long)N * N;
   const int gx = (int)std::min<long>((P / 2 + 255) / 256, 1024);
   return launch_k<k_p_planes<T>>(LF_KIND_PP, dim3(gx, B), 256, 0, st, reinterpret_cast<const T*>(a.phi),
-                                 reinterpret_cast<T*>(const_cast<void*>(a.pp)), P, 2 * nsteps + 1, t0, 0.5 * h);
+                                 reinterpret_cast<T*>(const_cast<void*>(a.pp)), P, 2 * nsteps + 1, t0, 0.5 * h, k0);
 }
 
 // The p planes hold p = M(t)^-1 grad(phi) at the 2n+1 times k / (2n), k = 0..2n, ascending; an
@@ -525,6 +525,36 @@ cudaError_t run_lens_cluster(const StageArgs& a, int B, int C, int nsteps, doubl
   return run_store_field<T>(spare, a.f_out, a.out_f64, (long)n, st);
 }
 
+// The lens without room for all p planes, two or three components of 256^2: step by step, with p at the step's three
+// times and the field between steps in the workspace's 4 C planes a map, which the clusters do not use.  The bits are
+// those of the lens with all p planes.  In the cluster kernel, once per component plane, p costs almost a stage.  us
+// per lens of n = 7 in passes, formed in the kernel and by steps: 1, 15, 32, 96 QU maps 325, 665, 1,094, 3,040; 232,
+// 708, 1,233, 3,536; 187, 524, 977, 2,719; float64, 1, 8, 32, 96 QU maps 360, 635, 2,388, 6,785; 258, 764, 2,576, 7,260;
+// 270, 725, 2,395, 6,754.  At 64^2 and 128^2 the launches cost more than that; with one component there is no room.
+template <typename T, int N, int C, bool ADJ>
+cudaError_t run_lens_steps(const StageArgs& a0, int B, int nsteps, double t0, double t1, cudaStream_t st) {
+  static_assert(C >= 2, "one field and six p planes");
+  constexpr int CL = cluster_blocks<N>(), io64 = std::is_same<T, double>::value;
+  const size_t n = (size_t)N * N * B * C;
+  StageArgs a = a0;
+  a.pp = static_cast<char*>(a0.y0) + sizeof(T) * n;
+  ClusterArgs c = cluster_args(a, B, C, 1, t0, (t1 - t0) / nsteps);
+  const bool staged = nsteps == 1 && clobbers(a.f_out, a.out_f64, a.f_in, a.in_f64, n);
+  for (int i = 0; i < nsteps; ++i) {
+    cudaError_t e = run_p_planes<T>(a, N, B, 1, 0.0, 1.0 / nsteps, st, 2 * (c.rev ? nsteps - 1 - i : i));
+    if (e != cudaSuccess) return e;
+    const bool out = i == nsteps - 1 && !staged;
+    c.f_out = out ? a.f_out : a.y0;
+    c.out_f64 = out ? a.out_f64 : io64;
+    e = launch_clusters<cluster_lens_kernel<T, N, ADJ, true>, CL>((long)B * C, ClGeo<T, N, CL>::NT,
+                                                                cluster_smem<T, N, CL>(), st, c);
+    if (e != cudaSuccess) return e;
+    c.f_in = a.y0;
+    c.in_f64 = io64;
+  }
+  return staged ? run_store_field<T>(a.y0, a.f_out, a.out_f64, (long)n, st) : cudaSuccess;
+}
+
 // One step of a reverse pass on clusters: p at the step's three times (float32; into ``pp``, along ``f``),
 // ``f`` (standard) and ``d`` (adjoint) side by side with their records, then the step's delta-phi terms.  Neither
 // system's output may share memory with what the other reads, nor its own but in place.
@@ -568,16 +598,11 @@ cudaError_t run_lens_n(const StageArgs& a, int B, int nsteps, double t0, double 
       }
       return run_lens_cluster<T, N, ADJ, true>(a, B, C, nsteps, t0, t1, a.y0, st);
     }
-    // p formed from the derivative planes costs a cluster almost a stage, once per component plane; the row pass
-    // forms it once per map.  256^2 QU, us per lens of n = 7 in passes and on clusters (14 at once), 24, 30, 64, 128
-    // and 192 planes: 520, 670, 1,101, 2,041, 3,049 and 496, 712, 1,246, 2,469, 3,555; adjoint 48, 64, 128 planes:
-    // 1,022, 1,227, 2,303 and 1,000, 1,291, 2,570.  T and TQU maps: within 5% of one another there.
-    auto passes_faster = [&](int clusters) {
-      return N == 256 && C == 2 && sizeof(T) == 4 && (long)B * C > (ADJ ? 4 : 2) * (long)clusters;
-    };
-    if (!a.pp) {
-      const int clusters = resident<T, N, cluster_lens_kernel<T, N, ADJ, false>>(st);
-      if (clusters && !passes_faster(clusters))
+    if constexpr (N == 256 && C >= 2) {
+      if (!a.pp && resident<T, N, cluster_lens_kernel<T, N, ADJ, true>>(st))
+        return run_lens_steps<T, N, C, ADJ>(a, B, nsteps, t0, t1, st);
+    } else {
+      if (!a.pp && resident<T, N, cluster_lens_kernel<T, N, ADJ, false>>(st))
         return run_lens_cluster<T, N, ADJ, false>(a, B, C, nsteps, t0, t1, a.y0, st);
     }
   }
@@ -838,13 +863,8 @@ cudaError_t run_vjp_n(const StageArgs& af0, const StageArgs& ad0, double* dacc, 
   StageArgs af = af0, ad = ad0;
   const double h = (t1 - t0) / nsteps;
   if constexpr (N <= 256) {
-    // Many float64 maps of 256^2 in two or three components keep the row passes' shared p faster than seven clusters
-    // at once.  ms in passes and on clusters, n = 7: QU, 64, 96, 192 planes 7.5, 10.9, 20.4 and 7.5, 11.1, 21.8; TQU,
-    // 45, 60, 96, 144 planes 5.3, 6.6, 9.7, 14.1 and 5.2, 6.8, 10.7, 15.9.
-    const int clusters = resident<T, N, cluster_step_kernel<T, N>>(st);
-    const bool passes_faster =
-        N == 256 && sizeof(T) == 8 && C >= 2 && (long)B * C > (C == 2 ? 12 : 8) * (long)clusters;
-    if (clusters && !passes_faster) return run_vjp_cluster<T, N, C>(af0, ad0, dacc, B, nsteps, t0, t1, st);
+    if (resident<T, N, cluster_step_kernel<T, N>>(st))
+      return run_vjp_cluster<T, N, C>(af0, ad0, dacc, B, nsteps, t0, t1, st);
   }
   const double hh = h / 2.0;
   const double cw[4] = {1.0, 2.0, 2.0, 1.0};

@@ -1148,12 +1148,12 @@ __global__ void __launch_bounds__(NT, MINB) k_row_rows(StageArgs a) {
 
 // ====================================================== p planes
 // p = M(t)^-1 grad(phi), M = I + t grad grad phi (lense_flow.py:373-381,
-// :398-415), at the K = 2n+1 stage times t_k = t0 + k hh of an RK4
+// :398-415), at the K = 2n+1 stage times t_k = t0 + (k0 + k) hh of an RK4
 // integration, from the five derivative planes; float64 arithmetic, stored in
 // T.  grid: x covers P/2 pixel pairs, y = map.
 template <typename T>
 __global__ void __launch_bounds__(256) k_p_planes(const T* __restrict__ planes, T* __restrict__ pp, long P, int K,
-                                                  double t0, double hh) {
+                                                  double t0, double hh, int k0) {
   const long map = blockIdx.y;
   const T* ph = planes + map * 5 * P;
   T* out = pp + map * (long)K * 2 * P;
@@ -1162,7 +1162,7 @@ __global__ void __launch_bounds__(256) k_p_planes(const T* __restrict__ planes, 
 #pragma unroll
     for (int j = 0; j < 5; ++j) f[j] = reinterpret_cast<const c2<T>*>(ph + j * P)[i];
     for (int k = 0; k < K; ++k) {
-      const double t = t0 + k * hh;
+      const double t = t0 + (k0 + k) * hh;
       double ox[2], oy[2];
       p_vector<double>(f[0].x, f[1].x, f[2].x, f[3].x, f[4].x, t, ox[0], oy[0]);
       p_vector<double>(f[0].y, f[1].y, f[2].y, f[3].y, f[4].y, t, ox[1], oy[1]);

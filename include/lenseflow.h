@@ -68,8 +68,9 @@ size_t lf_workspace_bytes(lf_plan_t plan, int batch, int adjoint);
  * 373-381, :398-415; two planes per time and map) so that every row pass
  * reads two planes per pixel instead of five.  lf_lense_flow takes that path
  * whenever ws_bytes is at least this; with at least lf_workspace_bytes it
- * forms p from the derivative planes in every stage: a caller that cannot get
- * this much falls back on that. */
+ * forms p from the derivative planes in every stage (N = 256 with two or three
+ * components: for one step at a time, with the same results bit for bit): a
+ * caller that cannot get this much falls back on that. */
 size_t lf_workspace_bytes_n(lf_plan_t plan, int batch, int adjoint, int nsteps);
 /* Bytes of the derivative-plane buffer for ``batch`` maps. */
 size_t lf_phi_planes_bytes(lf_plan_t plan, int batch);
