@@ -170,7 +170,10 @@ __device__ __forceinline__ void cluster_sync() {
 // runs out too: each waits once more at most (about two seconds with its drain), puts nothing after that and comes
 // here or has finished.  The barrier, which threads that have exited do not hold up, keeps every block's shared
 // memory until the last put into it has been sent and drained.
-__device__ __forceinline__ void cluster_leave() { cluster_sync(); }
+__device__ __forceinline__ void cluster_leave() {  // (not .aligned: reached by a branch)
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
 
 // ------------------------------------------------------ group transforms
 // One radix-R pass on registers: butterfly i of a lane is b = lane + TP i, its input r in register i + (E/R) r.
